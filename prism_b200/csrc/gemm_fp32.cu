@@ -2,84 +2,402 @@
 // A [M, K] row-major, W [N, K] row-major (the [out, in] layout of the model
 // file, andre-fu/prism engine/weight_pool.py:46-70; F.linear at
 // engine/executor.py:109,122,125,127,130).  CUDA-core FFMA only: no tensor
-// cores, no TF32, no split-K.  Every output element is accumulated over k in
-// ascending order inside one thread, so its value does not depend on M, on
-// the row's place in the batch, or on the grid.
+// cores, no TF32.
+//
+// Every kernel here adds an output's products in one order, which depends on
+// K alone: K is cut into slices of 32, slice c belongs to class c % 8, a class
+// is one chain of fused multiply-adds over its slices in ascending order, and
+// the eight classes' sums are added in ascending order.  So a value does not
+// depend on M, on the row's place in the batch, on the grid or on the kernel,
+// and a product can still be spread over eight threads (few rows: the lanes of
+// one warp) or eight CTAs (few tiles: a cluster) where one chain per output
+// would leave the GPU idle.
+//
+// Few rows (M <= 16) are bound by the stream of weights: measured at 3 rows,
+// K 896, N 151,936 (545 MB) 2.4 ms with one tile kernel for every M, 0.11 ms here.
 #include "common.cuh"
 
 namespace prism {
+namespace f32gemm {
 
-template <int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-sgemm_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
-                const void* __restrict__ bias, int bias_bf16, float* __restrict__ C, int ldc,
-                int M, int N, int K) {
+constexpr int SLICE = 32, CLASSES = 8, PERIOD = SLICE * CLASSES;
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// `bytes` of the 16 (of the 4) are copied, the rest of the destination becomes zero
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const float* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// ---- few rows -----------------------------------------------------------------------------------------
+// A CTA owns BN weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared
+// memory stages (cp.async; the weights of the first stages are asked for before the dependency wait where the
+// caller says that no earlier kernel of the stream writes them, w_static).  Thread =
+// (class, column group): the eight classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie
+// at (class, piece ^ class), so that the eight lanes read eight different bank groups.
+// BN 8 where N is small (N 896: 112 CTAs), else 32 with two columns a thread, which halves the reads of A.
+template <int MT, int BN, int CPT, int STAGES, bool VEC>
+__global__ void __launch_bounds__(BN / CPT * CLASSES)
+few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
+                int bias_bf16, float* C, int ldc, int M, int N, int K, int w_static) {
+    constexpr int THREADS = BN / CPT * CLASSES;
+    constexpr int STAGE = (BN + MT) * PERIOD;
+    extern __shared__ __align__(16) float smem[];
+    const int tid = threadIdx.x, j = tid % CLASSES, cg = tid / CLASSES;
+    const int n0 = blockIdx.x * BN;
+    const int periods = (K + PERIOD - 1) / PERIOD;
+
+    auto load = [&](const float* src, int ld, int rows, int limit, int row0, int period, float* dst) {
+        // rows x 64 pieces of 16 bytes
+        for (int idx = tid; idx < rows * (PERIOD / 4); idx += THREADS) {
+            const int r = idx / (PERIOD / 4), piece = idx % (PERIOD / 4);
+            const int cls = piece / 8, at = cls * 8 + ((piece % 8) ^ cls);
+            const int k = period * PERIOD + piece * 4;
+            const uint32_t d = smem_addr(dst + r * PERIOD + at * 4);
+            const int have = row0 + r < limit ? min(max(K - k, 0), 4) : 0;
+            const float* s = have ? src + (size_t)(row0 + r) * ld + k : src;
+            if (VEC) {
+                copy16(d, s, have * 4);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) copy4(d + 4 * e, e < have ? s + e : src, e < have ? 4 : 0);
+            }
+        }
+    };
+
     pdl_trigger();
-    pdl_wait();
-    constexpr int THREADS = (BM / TM) * (BN / TN);
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
+    if (!w_static) pdl_wait();
+    W = pdl_fresh(W);
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < periods) load(W, ldw, BN, N, n0, s, smem + s * STAGE);
+    if (w_static) pdl_wait();
+    A = pdl_fresh(A);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < periods) load(A, lda, MT, M, 0, s, smem + s * STAGE + BN * PERIOD);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int idx = tid; idx < BM * BK; idx += THREADS) {
-            const int r = idx / BK, c = idx % BK;
-            As[c][r] = (m0 + r < M && k0 + c < K) ? A[(size_t)(m0 + r) * lda + k0 + c] : 0.f;
-        }
-        for (int idx = tid; idx < BN * BK; idx += THREADS) {
-            const int r = idx / BK, c = idx % BK;
-            Ws[c][r] = (n0 + r < N && k0 + c < K) ? W[(size_t)(n0 + r) * ldw + k0 + c] : 0.f;
-        }
+    float acc[MT][CPT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int p = 0; p < CPT; ++p) acc[m][p] = 0.f;
+
+    for (int t = 0; t < periods; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        const int next = t + STAGES - 1;
+        if (next < periods) {
+            float* st = smem + (next % STAGES) * STAGE;
+            load(W, ldw, BN, N, n0, next, st);
+            load(A, lda, MT, M, 0, next, st + BN * PERIOD);
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float4* ws = reinterpret_cast<const float4*>(smem + (t % STAGES) * STAGE);
+        const float4* xs = ws + BN * (PERIOD / 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = j * 8 + (i ^ j);
+            float4 w[CPT];
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) w[p] = ws[(cg + p * (BN / CPT)) * (PERIOD / 4) + at];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float4 x = xs[m * (PERIOD / 4) + at];
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) {
+                    acc[m][p] = fmaf(x.x, w[p].x, acc[m][p]);
+                    acc[m][p] = fmaf(x.y, w[p].y, acc[m][p]);
+                    acc[m][p] = fmaf(x.z, w[p].z, acc[m][p]);
+                    acc[m][p] = fmaf(x.w, w[p].w, acc[m][p]);
+                }
+            }
+        }
     }
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = m0 + ty * TM + i;
-        if (m >= M) continue;
+    for (int m = 0; m < MT; ++m) {
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tx * TN + j;
-            if (n >= N) continue;
-            float v = acc[i][j];
-            if (bias != nullptr) v += load_param(bias, bias_bf16, n);
-            C[(size_t)m * ldc + n] = v;
+        for (int p = 0; p < CPT; ++p) {
+            float v = __shfl_sync(0xffffffffu, acc[m][p], 0, CLASSES);
+#pragma unroll
+            for (int c = 1; c < CLASSES; ++c) v += __shfl_sync(0xffffffffu, acc[m][p], c, CLASSES);
+            const int n = n0 + cg + p * (BN / CPT);
+            if ((m * CPT + p) % CLASSES == j && m < M && n < N) {
+                if (bias != nullptr) v += load_param(bias, bias_bf16, n);
+                C[(size_t)m * ldc + n] = v;
+            }
         }
     }
 }
 
+// ---- many rows --------------------------------------------------------------------------------------
+// BM x BN outputs a CTA, TM x TN a thread, one slice of K a step (the next one on its way in registers), the
+// multiply-adds in pairs of rows (fma.rn.f32x2).  SPLIT: the eight classes of a tile are the eight CTAs of a
+// cluster, whose sums meet through distributed shared memory; taken where the tiles alone would not fill the GPU.
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
+                 int bias_bf16, float* C, int ldc, int M, int N, int K) {
+    constexpr int THREADS = (BM / TM) * (BN / TN);
+    constexpr int LA = BM * 8 / THREADS, LW = BN * 8 / THREADS;      // 16-byte pieces of a slice a thread brings
+    static_assert(BM % 32 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN == 4 && LA * THREADS == BM * 8 && LW * THREADS == BN * 8, "");
+    struct Tiles {
+        float a[2][SLICE][BM];
+        float w[2][SLICE][BN];
+    };
+    __shared__ __align__(16) union {
+        Tiles t;
+        float sums[SPLIT ? BM : 1][SPLIT ? BN : 1];
+    } sm;
+    const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int slices = (K + SLICE - 1) / SLICE;
+    const int first = SPLIT ? (int)blockIdx.z : 0;                  // a cluster is (1, 1, 8): its rank is the class
+
+    pdl_trigger();
+    pdl_wait();
+    A = pdl_fresh(A);
+    W = pdl_fresh(W);
+
+    float4 ra[LA], rw[LW];
+    auto piece = [&](const float* src, int ld, int row, int limit, int k) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < limit && k < K) {
+            const float* s = src + (size_t)row * ld + k;
+            if (VEC && k + 4 <= K) {
+                v = *reinterpret_cast<const float4*>(s);
+            } else {
+                v.x = s[0];
+                if (k + 1 < K) v.y = s[1];
+                if (k + 2 < K) v.z = s[2];
+                if (k + 3 < K) v.w = s[3];
+            }
+        }
+        return v;
+    };
+    // neighbouring threads bring neighbouring rows: their transposed stores meet no bank twice
+    auto fetch = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < LA; ++i) {
+            const int idx = tid + i * THREADS;
+            ra[i] = piece(A, lda, m0 + idx % BM, M, c * SLICE + idx / BM * 4);
+        }
+#pragma unroll
+        for (int i = 0; i < LW; ++i) {
+            const int idx = tid + i * THREADS;
+            rw[i] = piece(W, ldw, n0 + idx % BN, N, c * SLICE + idx / BN * 4);
+        }
+    };
+    auto put = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < LA; ++i) {
+            const int idx = tid + i * THREADS, r = idx % BM, k = idx / BM * 4;
+            sm.t.a[b][k][r] = ra[i].x, sm.t.a[b][k + 1][r] = ra[i].y, sm.t.a[b][k + 2][r] = ra[i].z, sm.t.a[b][k + 3][r] = ra[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < LW; ++i) {
+            const int idx = tid + i * THREADS, r = idx % BN, k = idx / BN * 4;
+            sm.t.w[b][k][r] = rw[i].x, sm.t.w[b][k + 1][r] = rw[i].y, sm.t.w[b][k + 2][r] = rw[i].z, sm.t.w[b][k + 3][r] = rw[i].w;
+        }
+    };
+
+    uint64_t acc[TM / 2][TN];                      // two rows each
+    float total[SPLIT ? 1 : TM][SPLIT ? 1 : TN];
+#pragma unroll
+    for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+        for (int q = 0; q < TN; ++q) acc[i][q] = 0;
+    for (auto& t : total)
+        for (auto& v : t) v = 0.f;
+    int b = 0, cls = first, c = first;
+    // the slice after c in this CTA's order; the classes of an unsplit tile follow one another
+    auto after = [&](int& cl, int s) {
+        s += CLASSES;
+        while (!SPLIT && s >= slices && ++cl < CLASSES) s = cl;
+        return s;
+    };
+    auto close = [&](int cl) {                     // the sums of class cl are complete
+        if constexpr (!SPLIT) {
+#pragma unroll
+            for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+                for (int q = 0; q < TN; ++q) {
+                    const float2 v = unpack2(acc[i][q]);
+                    total[2 * i][q] = cl == 0 ? v.x : total[2 * i][q] + v.x;
+                    total[2 * i + 1][q] = cl == 0 ? v.y : total[2 * i + 1][q] + v.y;
+                    acc[i][q] = 0;
+                }
+        }
+    };
+    if (c < slices) {
+        fetch(c);
+        put(0);
+        __syncthreads();
+        while (true) {
+            int ncls = cls;
+            const int nc = after(ncls, c);
+            const bool more = nc < slices;
+            if (more) fetch(nc);
+#pragma unroll
+            for (int k = 0; k < SLICE; ++k) {
+                ulonglong2 a[TM / 4];
+#pragma unroll
+                for (int i = 0; i < TM / 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(&sm.t.a[b][k][ty * 4 + i * (BM / (TM / 4))]);
+                const float4 w = *reinterpret_cast<const float4*>(&sm.t.w[b][k][tx * 4]);
+                const uint64_t w2[4] = {pack2(w.x, w.x), pack2(w.y, w.y), pack2(w.z, w.z), pack2(w.w, w.w)};
+#pragma unroll
+                for (int i = 0; i < TM / 4; ++i)
+#pragma unroll
+                    for (int q = 0; q < TN; ++q) {
+                        fma2(acc[2 * i][q], a[i].x, w2[q]);
+                        fma2(acc[2 * i + 1][q], a[i].y, w2[q]);
+                    }
+            }
+            if (!SPLIT && (!more || ncls != cls))
+                for (int cl = cls; cl < (more ? ncls : CLASSES); ++cl) close(cl);      // empty classes add their zero too
+            if (!more) break;
+            put(b ^ 1);
+            __syncthreads();
+            b ^= 1, c = nc, cls = ncls;
+        }
+    }
+    // row of accumulator i (pairs lie in groups of four rows)
+    auto row = [&](int i) { return ty * 4 + i / 4 * (BM / (TM / 4)) + i % 4; };
+    if constexpr (!SPLIT) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + row(i);
+            if (m >= M) continue;
+#pragma unroll
+            for (int q = 0; q < TN; ++q) {
+                const int n = n0 + tx * 4 + q;
+                if (n >= N) continue;
+                float v = total[i][q];
+                if (bias != nullptr) v += load_param(bias, bias_bf16, n);
+                C[(size_t)m * ldc + n] = v;
+            }
+        }
+    } else {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+            for (int q = 0; q < TN; ++q) {
+                const float2 v = unpack2(acc[i][q]);
+                sm.sums[row(2 * i)][tx * 4 + q] = v.x;
+                sm.sums[row(2 * i + 1)][tx * 4 + q] = v.y;
+            }
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+        // this CTA adds up an eighth of the tile's rows
+        for (int idx = tid; idx < BM / CLASSES * BN; idx += THREADS) {
+            const int r = first * (BM / CLASSES) + idx / BN, n = idx % BN;
+            float v = 0.f;
+#pragma unroll
+            for (int cl = 0; cl < CLASSES; ++cl) {
+                uint32_t remote;
+                float x;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&sm.sums[r][n])), "r"(cl));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
+                v = cl == 0 ? x : v + x;
+            }
+            if (m0 + r < M && n0 + n < N) {
+                if (bias != nullptr) v += load_param(bias, bias_bf16, n0 + n);
+                C[(size_t)(m0 + r) * ldc + n0 + n] = v;
+            }
+        }
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    }
+}
+
+struct Call {
+    const float* A;
+    int lda;
+    const float* W;
+    int ldw;
+    const void* bias;
+    int bb;
+    float* C;
+    int ldc, M, N, K, w_static;
+    cudaStream_t stream;
+};
+
+template <int MT, int BN, int CPT, int STAGES, bool VEC> int few(const Call& c) {
+    constexpr int smem = STAGES * (BN + MT) * PERIOD * 4;
+    auto kern = few_rows_kernel<MT, BN, CPT, STAGES, VEC>;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return (int)launch_kernel(kern, dim3((c.N + BN - 1) / BN), dim3(BN / CPT * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
+                              c.bb, c.C, c.ldc, c.M, c.N, c.K, c.w_static);
+}
+
+// BN 8 keeps every SM busy down to N of about a thousand; from 148 x 32 columns on wider CTAs fill the GPU too
+template <int MT, bool VEC> int few_n(const Call& c) {
+    return c.N >= 4736 ? few<MT, 32, 2, 3, VEC>(c) : few<MT, 8, 1, 5, VEC>(c);
+}
+
+template <bool VEC> int few_m(const Call& c) {
+    if (c.M <= 1) return few_n<1, VEC>(c);
+    if (c.M <= 2) return few_n<2, VEC>(c);
+    if (c.M <= 4) return few_n<4, VEC>(c);
+    if (c.M <= 8) return few_n<8, VEC>(c);
+    return few_n<16, VEC>(c);
+}
+
+template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC> int many(const Call& c) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((c.N + BN - 1) / BN, (c.M + BM - 1) / BM, SPLIT ? CLASSES : 1);
+    cfg.blockDim = dim3((BM / TM) * (BN / TN));
+    cfg.stream = c.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = SPLIT ? CLASSES : 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, many_rows_kernel<BM, BN, TM, TN, SPLIT, VEC>, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C, c.ldc, c.M,
+                                   c.N, c.K);
+}
+
+template <bool VEC> int pick(const Call& c) {
+    if (c.M <= 16) return few_m<VEC>(c);
+    // tiles of 64 x 64 that do not fill the 148 SMs twice have their K shared by a cluster
+    const long tiles = (long)((c.M + 63) / 64) * ((c.N + 63) / 64);
+    if (tiles < 296) return many<64, 64, 4, 4, true, VEC>(c);
+    if (c.M <= 64) return many<64, 64, 4, 4, false, VEC>(c);
+    return many<128, 64, 8, 4, false, VEC>(c);
+}
+
+}  // namespace f32gemm
 }  // namespace prism
 
 PRISM_EXPORT int prism_sgemm_nt(const float* A, int lda, const float* W, int ldw, const void* bias,
-                                int bias_dtype, float* C, int ldc, int M, int N, int K,
+                                int bias_dtype, float* C, int ldc, int M, int N, int K, int w_static,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    const int bb = bias_dtype == PRISM_DTYPE_BF16;
-    if (M <= 16) {
-        dim3 grid((N + 63) / 64, (M + 15) / 16);
-        prism::sgemm_nt_kernel<16, 64, 32, 1, 4><<<grid, 256, 0, stream>>>(A, lda, W, ldw, bias, bb, C, ldc, M, N, K);
-    } else {
-        dim3 grid((N + 63) / 64, (M + 63) / 64);
-        prism::sgemm_nt_kernel<64, 64, 16, 4, 4><<<grid, 256, 0, stream>>>(A, lda, W, ldw, bias, bb, C, ldc, M, N, K);
-    }
-    return (int)cudaPeekAtLastError();
+    const prism::f32gemm::Call c{A, lda, W, ldw, bias, bias_dtype == PRISM_DTYPE_BF16, C, ldc, M, N, K, w_static, stream};
+    // 16-byte copies where every row starts on a 16-byte boundary
+    const bool vec = ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && (M == 1 || lda % 4 == 0) && (N == 1 || ldw % 4 == 0);
+    return vec ? prism::f32gemm::pick<true>(c) : prism::f32gemm::pick<false>(c);
 }

@@ -169,6 +169,25 @@ def test_sgemm(M, N, K):
     assert torch.equal(out1[0], out[M // 2])
 
 
+@pytest.mark.parametrize("N,K", [(7, 5), (896, 864), (130, 257), (4736, 300), (9000, 64)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_sgemm_same_at_every_row_count(N, K, pad):
+    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone; 16-byte and single
+    copies) adds a row's products in the same order.  Bound: K products of about 0.05, the chains at most K / 8 long."""
+    ops = _ops()
+    x = _rand((300, K + pad), torch.float32, 6)[:, :K]
+    w = _rand((N, K + pad), torch.float32, 7, 0.05)[:, pad:]
+    b = _rand((N,), torch.float32, 8)
+    ref = x.double() @ w.double().T + b.double()
+    rows = None
+    for M in (300, 129, 65, 64, 17, 16, 9, 8, 5, 4, 3, 2, 1):
+        out = torch.full((M, N + pad), 7.0, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[300 - M:], w, b, out[:, :N])
+        rows = out if rows is None else rows
+        assert torch.equal(out, rows[300 - M:]), M                       # the column behind the last stays as it was
+    assert (rows[:, :N].double() - ref).abs().max() < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 152, 96), (8, 4608, 3584), (300, 1000, 512)])
 def test_linear_bf16(M, N, K):
     ops = _ops()
