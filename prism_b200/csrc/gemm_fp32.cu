@@ -15,7 +15,7 @@
 //
 // Few rows (M <= 16) are bound by the stream of weights: measured at 3 rows,
 // K 896, N 151,936 (545 MB) 2.4 ms with one tile kernel for every M, 0.11 ms here.
-#include "common.cuh"
+#include "f32x2.cuh"
 
 namespace prism {
 namespace f32gemm {
@@ -139,20 +139,6 @@ few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __
 // BM x BN outputs a CTA, TM x TN a thread, one slice of K a step (the next one on its way in registers), the
 // multiply-adds in pairs of rows (fma.rn.f32x2).  SPLIT: the eight classes of a tile are the eight CTAs of a
 // cluster, whose sums meet through distributed shared memory; taken where the tiles alone would not fill the GPU.
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
 template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,

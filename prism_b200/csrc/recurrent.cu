@@ -33,6 +33,7 @@
 //   * prism_headnorm_gate    o / rms(o) per head, times a weight, times silu(gate), times a constant;
 //   * prism_part_norm_gate   the same over equal parts of the concatenated heads, the gate before or after the norm;
 //   * prism_step_sizes       softplus(z + bias) and the decay exp(-exp(a_log) times it) per head and token.
+#include "f32x2.cuh"
 #include "mma_helpers.cuh"
 
 #define PRISM_SCAN_DELTA 0
@@ -350,15 +351,24 @@ __global__ void part_norm_gate_kernel(const float* __restrict__ x_in, const floa
 
 // ---------------------------------------------------------------------------------------------------------
 // The scan.  grid (heads, segments, column blocks); the L threads of a column are neighbouring lanes of a warp,
-// each owns R rows of that column of S in registers - quads of four neighbouring rows, quad part + L m - and
-// they add up their partial dot products by shuffles.  The step's vectors come through shared memory TB tokens
-// at a time with cp.async, the next block on its way while this one is worked on; a thread reads its quads
-// of q, k (w, u) with 128-bit loads.  The state is kept in memory as [slot][head][column][row], so that the
-// threads of a column read neighbouring floats.
+// each owns R rows - quads of four neighbouring rows, quad part + L m - of CPT neighbouring columns of S in
+// registers, and they add up their partial dot products by shuffles.  The step's vectors come through shared memory
+// TB tokens at a time with cp.async, the next blocks on their way while this one is worked on; a thread reads its
+// quads of q, k (w, e, c) with 128-bit loads, once for its CPT columns.  The state is kept in memory as
+// [slot][head][column][row], so that the threads of a column read neighbouring floats.
+//
+// What bounds it, and the split: a token's work on a column is a chain (the delta rules: dot product, shuffles,
+// update), so few columns leave latency exposed; and every column of a thread wants the token's vectors through
+// shared memory, 128 bytes a cycle and SM, so many columns are bound by that unless a thread has several.  Tokens are
+// taken eight at a time in straight line code: a token's read-out stands behind the next one's dot products, where
+// the chain waits for its shuffles, and the eight read-outs are added up across the lanes together (7 shuffles
+// instead of 24; the additions are the same).  The results do not depend on CPT, on the blocks or on how a request
+// was cut: every sum has one order.
 //   SCAN_DELTA:  x [T, *] row stride xs: q of kv head g at qo + g dk, k at ko + g dk; v at vo + h dv;
 //                bg [T, 2 H]: beta | g.
 //   SCAN_BONUS:  r at qo + h dk, k at ko + h dk, v at vo + h dv, the decay's exponent ww [T, H dk] (row stride ws)
-//                with w = exp(-exp(ww + w0)) formed in shared memory, w0 [H dk], bonus u [H dk].
+//                with w = exp(-exp(ww + w0)) formed in shared memory, w0 [H dk], bonus u [H dk].  The bonus term is
+//                (sum_i r_i u_i k_i) v: one sum for all columns.
 //   SCAN_CHANNEL: q, k, v as for SCAN_DELTA; the decay itself in ww [T, H dk] (row stride ws); bg [T, H]: beta.
 //   SCAN_GENERAL: r, k, v as for SCAN_BONUS; the decay itself in ww; ex [T, 2 H dk]: the unit key e at h dk, c at (H + h) dk.
 //   SCAN_RETAIN: q, k, v as for SCAN_BONUS; the decay of head h in w0[h].
@@ -382,7 +392,7 @@ struct ScanArgs {
     const int* seg_start;
     const int* slots;
     float* out;              // [T, H, dv]
-    int H, rep, dk, dkp, dv, cols, colsp, L, TB;
+    int H, rep, dk, dkp, dv, cols, colsp, L, TB, NBUF;
     int vec;                 // every source row piece starts on 16 bytes and is whole quads long
     int w_ready;             // BONUS: ww holds the decay itself already (prism_decay_from_exponent)
 };
@@ -391,6 +401,19 @@ __device__ __forceinline__ void cp_async_f(float* smem, const float* gmem, int f
     const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
     if (floats == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gmem));
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(gmem));
+}
+
+// all but the newest `n` groups (at most 6) have landed
+__device__ __forceinline__ void cp_async_wait_upto(int n) {
+    switch (n) {
+        case 1: cp_async_wait<1>(); break;
+        case 2: cp_async_wait<2>(); break;
+        case 3: cp_async_wait<3>(); break;
+        case 4: cp_async_wait<4>(); break;
+        case 5: cp_async_wait<5>(); break;
+        case 6: cp_async_wait<6>(); break;
+        default: cp_async_wait<0>();
+    }
 }
 
 // sum over the L (a power of two, known when the kernel is compiled) neighbouring lanes that share a column
@@ -408,8 +431,24 @@ __host__ __device__ constexpr int scan_vectors(int mode) {
     return (mode == PRISM_SCAN_DELTA || mode == PRISM_SCAN_RETAIN || mode == PRISM_SCAN_TOKEN) ? 2 : (mode == PRISM_SCAN_GENERAL ? 5 : 3);
 }
 
-template <int MODE, int R, int L>
-__global__ void scan_kernel(const ScanArgs a) {
+// four neighbouring floats of shared memory as two pairs
+__device__ __forceinline__ ulonglong2 quad(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+// x . y over a thread's quads, four chains side by side
+template <int Q> __device__ __forceinline__ float quad_dot(const uint64_t (&x)[2 * Q], const ulonglong2 (&y)[Q]) {
+    uint64_t a = 0, b = 0;
+#pragma unroll
+    for (int m = 0; m < Q; ++m) {
+        fma2(a, x[2 * m], y[m].x);
+        fma2(b, x[2 * m + 1], y[m].y);
+    }
+    const float2 p = unpack2(a), r = unpack2(b);
+    return (p.x + p.y) + (r.x + r.y);
+}
+
+// LONG: groups of eight tokens, with the registers that their straight line code wants; else (a few tokens a request,
+// bound by the state's way in and out) token by token, with as many CTAs on an SM as keep that busy.
+template <int MODE, int R, int L, int CPT, bool LONG>
+__global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel(const ScanArgs a) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -426,13 +465,12 @@ __global__ void scan_kernel(const ScanArgs a) {
     const int CT = blockDim.x - 32;
     const bool producer = (int)threadIdx.x >= CT;
     const int part = threadIdx.x % L;
-    const bool live = !producer && (int)threadIdx.x / L < ncols;
-    const int lc = live ? threadIdx.x / L : 0, col = col0 + lc;
+    const bool live = !producer && (int)threadIdx.x / L * CPT < ncols;      // CPT > 1: the columns are whole groups of CPT
+    const int lc = live ? threadIdx.x / L * CPT : 0, col = col0 + lc;
     const int kvh = h / a.rep;                         // DELTA: the q/k head this head uses
-    // shared, per token of a block:  first[dkp] (q or r) | second[dkp] (k) | third[dkp] (BONUS: w) | v[colsp] | 4 scalars
+    // shared, per token of a block:  first[dkp] (q or r) | second[dkp] (k) | further vectors [dkp] | v[colsp] | 4 scalars
     const int per_tok = NV * dkp + a.colsp + 4;
-    constexpr int NBUF = 3;                            // blocks of tokens in shared memory: in use, landed, on its way
-    float* ub = sm + (size_t)NBUF * TB * per_tok;      // BONUS: u[dkp]
+    const int NBUF = a.NBUF;                           // blocks of tokens in shared memory: one in use, the others landed or on their way
     const float* x = pdl_fresh(a.x);
     const float* bg = pdl_fresh(a.bg);
     const float* ww = pdl_fresh(a.ww);
@@ -450,43 +488,81 @@ __global__ void scan_kernel(const ScanArgs a) {
             sm[(size_t)slot * per_tok + at] = 0.f;
         }
     }
-    if (MODE == PRISM_SCAN_BONUS)
-        for (int i = threadIdx.x; i < dkp; i += blockDim.x) ub[i] = i < dk ? load_param(a.u, a.u_bf16, (size_t)h * dk + i) : 0.f;
     __syncthreads();
 
-    // the producer warp asks for block b0 of the segment's tokens into buffer `buf` ...
+    // the producer warp asks for block b0 of the segment's tokens into buffer `buf`: the lanes are dealt out to the
+    // pieces of a token's vectors, and where those are fewer than 32 to several tokens, so that a vector of a token
+    // costs an instruction or less ...
+    const int unit = a.vec ? 4 : 1;
+    const int nk = (dk + unit - 1) / unit, nc = (ncols + unit - 1) / unit;          // pieces per vector
+    const int lane = threadIdx.x & 31;
+    const int ktoks = nk <= 16 ? 32 / nk : 1, ctoks = nc <= 16 ? 32 / nc : 1;        // tokens side by side
+    const int kt = ktoks > 1 ? lane / nk : 0, kc = lane - kt * nk;
+    const int ct = ctoks > 1 ? lane / nc : 0, cc = lane - ct * nc;
+    const bool one_piece = a.vec && nk <= 32;          // a lane brings one piece of a vector at most
+    const size_t head_q = (size_t)((MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_CHANNEL || MODE == PRISM_SCAN_TOKEN) ? kvh : h) * dk;
     auto stage = [&](int b0, int buf) {
-        const int lane = threadIdx.x - CT;
         const int nb = min(TB, qlen - b0);
         float* dst0 = sm + (size_t)buf * TB * per_tok;
-        const int unit = a.vec ? 4 : 1;
-        const int nk = (dk + unit - 1) / unit, nc = (ncols + unit - 1) / unit;     // pieces per vector
-        const size_t head_q = (size_t)((MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_CHANNEL || MODE == PRISM_SCAN_TOKEN) ? kvh : h) * dk;
-        for (int tt = 0; tt < nb; ++tt) {
-            const size_t t = (size_t)(s0 + b0 + tt);
-            const float* xr = x + t * a.xs;
-            float* dst = dst0 + (size_t)tt * per_tok;
-            for (int c = lane; c < nk; c += 32) {
-                cp_async_f(dst + c * unit, xr + a.qo + head_q + c * unit, unit);
-                cp_async_f(dst + dkp + c * unit, xr + a.ko + head_q + c * unit, unit);
-                if (NV > 2) cp_async_f(dst + 2 * dkp + c * unit, ww + t * a.ws + (size_t)h * dk + c * unit, unit);
-                if (MODE == PRISM_SCAN_GENERAL) {
-                    cp_async_f(dst + 3 * dkp + c * unit, ex + t * a.es + (size_t)h * dk + c * unit, unit);
-                    cp_async_f(dst + 4 * dkp + c * unit, ex + t * a.es + (size_t)(a.H + h) * dk + c * unit, unit);
+        const size_t t = (size_t)(s0 + b0 + kt);
+        const float* xq = x + t * a.xs + head_q + a.qo + kc * unit;
+        const float* xk = x + t * a.xs + head_q + a.ko + kc * unit;
+        const float* wr = NV > 2 ? ww + t * a.ws + (size_t)h * dk + kc * unit : nullptr;
+        const float* er = NV > 3 ? ex + t * a.es + (size_t)h * dk + kc * unit : nullptr;
+        const size_t c_at = NV > 3 ? (size_t)a.H * dk : 0;                            // from the unit key to what it removes
+        const size_t xstep = (size_t)ktoks * a.xs, wstep = (size_t)ktoks * a.ws, estep = (size_t)ktoks * a.es;
+        float* dst = dst0 + (size_t)kt * per_tok + kc * unit;
+        if (one_piece) {
+            if (kt < ktoks && kc < nk)
+#pragma unroll 4
+                for (int tt = kt; tt < nb; tt += ktoks) {
+                    cp_async_f(dst, xq, 4);
+                    cp_async_f(dst + dkp, xk, 4);
+                    if (NV > 2) cp_async_f(dst + 2 * dkp, wr, 4);
+                    if (NV > 3) {
+                        cp_async_f(dst + 3 * dkp, er, 4);
+                        cp_async_f(dst + 4 * dkp, er + c_at, 4);
+                        er += estep;
+                    }
+                    xq += xstep, xk += xstep;
+                    if (NV > 2) wr += wstep;
+                    dst += ktoks * per_tok;
                 }
+        } else if (kt < ktoks) {
+            for (int tt = kt; tt < nb; tt += ktoks) {
+                for (int c = 0; c + kc < nk; c += 32) {
+                    cp_async_f(dst + c * unit, xq + c * unit, unit);
+                    cp_async_f(dst + dkp + c * unit, xk + c * unit, unit);
+                    if (NV > 2) cp_async_f(dst + 2 * dkp + c * unit, wr + c * unit, unit);
+                    if (NV > 3) {
+                        cp_async_f(dst + 3 * dkp + c * unit, er + c * unit, unit);
+                        cp_async_f(dst + 4 * dkp + c * unit, er + c_at + c * unit, unit);
+                    }
+                }
+                xq += xstep, xk += xstep;
+                if (NV > 2) wr += wstep;
+                if (NV > 3) er += estep;
+                dst += ktoks * per_tok;
             }
-            for (int c = lane; c < nc; c += 32)
-                cp_async_f(dst + NV * dkp + c * unit, xr + a.vo + (size_t)h * dv + col0 + c * unit, unit);
-            if ((MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_TOKEN) && lane < 2)  // beta (or dt), then g
-                cp_async_f(dst + NV * dkp + a.colsp + lane, bg + t * 2 * a.H + (size_t)lane * a.H + h, 1);
-            if (MODE == PRISM_SCAN_CHANNEL && lane == 0)                             // beta
-                cp_async_f(dst + NV * dkp + a.colsp, bg + t * a.H + h, 1);
+        }
+        if (ct < ctoks)
+            for (int tt = ct; tt < nb; tt += ctoks)
+                for (int c = cc; c < nc; c += 32)
+                    cp_async_f(dst0 + (size_t)tt * per_tok + NV * dkp + c * unit,
+                               x + (size_t)(s0 + b0 + tt) * a.xs + a.vo + (size_t)h * dv + col0 + c * unit, unit);
+        for (int tt = lane; tt < nb; tt += 32) {
+            float* sc = dst0 + (size_t)tt * per_tok + NV * dkp + a.colsp;
+            const size_t ts = (size_t)(s0 + b0 + tt);
+            if (MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_TOKEN) {              // beta (or dt), then g
+                cp_async_f(sc, bg + ts * 2 * a.H + h, 1);
+                cp_async_f(sc + 1, bg + ts * 2 * a.H + a.H + h, 1);
+            }
+            if (MODE == PRISM_SCAN_CHANNEL) cp_async_f(sc, bg + ts * a.H + h, 1);    // beta
         }
         cp_async_commit();
     };
     // ... and, once the copies of that block have landed (the caller has waited), turns the decay's exponent into the decay
     auto finish = [&](int b0, int buf) {
-        const int lane = threadIdx.x - CT;
         const int nb = min(TB, qlen - b0);
         float* dst0 = sm + (size_t)buf * TB * per_tok;
         __syncwarp();
@@ -499,24 +575,40 @@ __global__ void scan_kernel(const ScanArgs a) {
         }
     };
 
-    float S[R];
+    uint64_t S[CPT][R / 2], bonus[MODE == PRISM_SCAN_BONUS ? R / 2 : 1];
     float* st = a.state + (((size_t)a.slots[seg] * a.H + h) * dv + col) * dk;
     if (producer) {
-        stage(0, 0);
-        if (TB < qlen) stage(TB, 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
+        for (int i = 0; i < NBUF - 1; ++i) {
+            if (i * TB < qlen) stage(i * TB, i);
+            else cp_async_commit();
+        }
+        cp_async_wait_upto(NBUF - 2);
         finish(0, 0);
     } else {
 #pragma unroll
         for (int m = 0; m < Q; ++m) {
             const int i = 4 * (part + L * m);
-            if (live && a.vec && i + 3 < dk) {
-                const float4 v = *reinterpret_cast<const float4*>(st + i);
-                S[4 * m] = v.x; S[4 * m + 1] = v.y; S[4 * m + 2] = v.z; S[4 * m + 3] = v.w;
-            } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) S[4 * m + j] = (live && i + j < dk) ? st[i + j] : 0.f;
+            for (int p = 0; p < CPT; ++p) {
+                const float* sp = st + (size_t)p * dk + i;
+                if (live && a.vec && i + 3 < dk) {
+                    const float4 v = *reinterpret_cast<const float4*>(sp);
+                    S[p][2 * m] = pack2(v.x, v.y);
+                    S[p][2 * m + 1] = pack2(v.z, v.w);
+                } else {
+                    float v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[j] = (live && i + j < dk) ? sp[j] : 0.f;
+                    S[p][2 * m] = pack2(v[0], v[1]);
+                    S[p][2 * m + 1] = pack2(v[2], v[3]);
+                }
+            }
+            if (MODE == PRISM_SCAN_BONUS) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = i + j < dk ? load_param(a.u, a.u_bf16, (size_t)h * dk + i + j) : 0.f;
+                bonus[2 * m % (R / 2)] = pack2(v[0], v[1]);
+                bonus[(2 * m + 1) % (R / 2)] = pack2(v[2], v[3]);
             }
         }
     }
@@ -524,175 +616,196 @@ __global__ void scan_kernel(const ScanArgs a) {
     const float keep = MODE == PRISM_SCAN_RETAIN ? load_param(a.w0, a.w0_bf16, h) : 0.f;      // the head's constant decay
     const float skip = MODE == PRISM_SCAN_TOKEN && a.w0 != nullptr ? load_param(a.w0, a.w0_bf16, h) : 0.f;
 
+    auto read = [&](const ulonglong2 (&q)[Q], float (&o)[CPT]) {
+        if (MODE == PRISM_SCAN_BONUS) return;
+#pragma unroll
+        for (int p = 0; p < CPT; ++p) o[p] = quad_dot<Q>(S[p], q);
+    };
+    // One token, whose vectors lie at f1: S moves on, and q is what reads it out (`read`: this thread's part of column p),
+    // or, for the decayed sum with a bonus, o is read out at once.  `before`: the read-out of the token before (last_q
+    // into last_o) is still due; it stands where the chain waits for its shuffles.
+    auto token = [&](const float* f1, ulonglong2 (&q)[Q], float (&o)[CPT], bool before, const ulonglong2 (&last_q)[Q], float (&last_o)[CPT]) {
+        const float* row = f1 + 4 * part;
+        const float* vv = f1 + NV * dkp;
+        ulonglong2 k[Q];
+        float v[CPT];
+#pragma unroll
+        for (int m = 0; m < Q; ++m) k[m] = quad(row + dkp + 4 * L * m);
+#pragma unroll
+        for (int m = 0; m < Q; ++m) q[m] = quad(row + 4 * L * m);
+        if (CPT == 4) {
+            const float4 v4 = *reinterpret_cast<const float4*>(vv + lc);
+            v[0] = v4.x, v[1 % CPT] = v4.y, v[2 % CPT] = v4.z, v[3 % CPT] = v4.w;
+        } else if (CPT == 2) {
+            const float2 v2 = *reinterpret_cast<const float2*>(vv + lc);
+            v[0] = v2.x, v[1 % CPT] = v2.y;
+        } else {
+            v[0] = vv[lc];
+        }
+        if (MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_CHANNEL) {
+            const float beta = vv[a.colsp], g = MODE == PRISM_SCAN_DELTA ? vv[a.colsp + 1] : 1.f;
+            if (MODE == PRISM_SCAN_CHANNEL) {
+                if (before) read(last_q, last_o);      // S is about to decay
+#pragma unroll
+                for (int m = 0; m < Q; ++m) {
+                    const ulonglong2 w = quad(row + 2 * dkp + 4 * L * m);
+#pragma unroll
+                    for (int p = 0; p < CPT; ++p) {
+                        S[p][2 * m] = mul2(S[p][2 * m], w.x);
+                        S[p][2 * m + 1] = mul2(S[p][2 * m + 1], w.y);
+                    }
+                }
+            }
+            const uint64_t g2 = pack2(g, g);
+            float ks[CPT];
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) ks[p] = quad_dot<Q>(S[p], k);
+            if (MODE == PRISM_SCAN_DELTA && before) read(last_q, last_o);
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) ks[p] = column_sum<L>(ks[p]);
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) {
+                const float uu = MODE == PRISM_SCAN_DELTA ? beta * (v[p] - g * ks[p]) : beta * (v[p] - ks[p]);
+                const uint64_t u2 = pack2(uu, uu);
+#pragma unroll
+                for (int m = 0; m < Q; ++m) {
+                    if (MODE == PRISM_SCAN_DELTA) {
+                        S[p][2 * m] = mul2(S[p][2 * m], g2);
+                        S[p][2 * m + 1] = mul2(S[p][2 * m + 1], g2);
+                    }
+                    fma2(S[p][2 * m], k[m].x, u2);
+                    fma2(S[p][2 * m + 1], k[m].y, u2);
+                }
+            }
+        } else if (MODE == PRISM_SCAN_GENERAL) {
+            float es[CPT];                             // e^T S of a column, from the state before the token
+            {
+                ulonglong2 e[Q];
+#pragma unroll
+                for (int m = 0; m < Q; ++m) e[m] = quad(row + 3 * dkp + 4 * L * m);
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) es[p] = quad_dot<Q>(S[p], e);
+            }
+            if (before) read(last_q, last_o);
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) es[p] = column_sum<L>(es[p]);
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+                const ulonglong2 w = quad(row + 2 * dkp + 4 * L * m), c = quad(row + 4 * dkp + 4 * L * m);
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) {
+                    const uint64_t v2 = pack2(v[p], v[p]), e2 = pack2(-es[p], -es[p]);
+                    S[p][2 * m] = mad2(w.x, S[p][2 * m], mul2(k[m].x, v2));
+                    S[p][2 * m + 1] = mad2(w.y, S[p][2 * m + 1], mul2(k[m].y, v2));
+                    fma2(S[p][2 * m], c.x, e2);
+                    fma2(S[p][2 * m + 1], c.y, e2);
+                }
+            }
+        } else if (MODE == PRISM_SCAN_BONUS) {
+            uint64_t b0 = 0, b1 = 0;
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+                fma2(b0, mul2(q[m].x, bonus[2 * m % (R / 2)]), k[m].x);
+                fma2(b1, mul2(q[m].y, bonus[(2 * m + 1) % (R / 2)]), k[m].y);
+            }
+            const float2 p0 = unpack2(b0), p1 = unpack2(b1);
+            const float now = (p0.x + p0.y) + (p1.x + p1.y);
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) o[p] = fmaf(now, v[p], quad_dot<Q>(S[p], q));
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+                const ulonglong2 w = quad(row + 2 * dkp + 4 * L * m);
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) {
+                    const uint64_t v2 = pack2(v[p], v[p]);
+                    S[p][2 * m] = mad2(w.x, S[p][2 * m], mul2(k[m].x, v2));
+                    S[p][2 * m + 1] = mad2(w.y, S[p][2 * m + 1], mul2(k[m].y, v2));
+                }
+            }
+        } else {                                       // S <- (decay) S + k v^T, read out after it
+            const float dt = MODE == PRISM_SCAN_TOKEN ? vv[a.colsp] : 1.f;
+            const float g = MODE == PRISM_SCAN_TOKEN ? vv[a.colsp + 1] : keep;
+            const uint64_t g2 = pack2(g, g);
+            if (before) read(last_q, last_o);
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+                ulonglong2 w = make_ulonglong2(g2, g2);
+                if (MODE == PRISM_SCAN_GATED) w = quad(row + 2 * dkp + 4 * L * m);
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) {
+                    const float t = MODE == PRISM_SCAN_TOKEN ? dt * v[p] : v[p];
+                    const uint64_t v2 = pack2(t, t);
+                    S[p][2 * m] = mad2(w.x, S[p][2 * m], mul2(k[m].x, v2));
+                    S[p][2 * m + 1] = mad2(w.y, S[p][2 * m + 1], mul2(k[m].y, v2));
+                }
+            }
+        }
+    };
+    // token tt of the segment, whose vectors lie at f1
+    auto store = [&](int tt, const float* f1, float (&o)[CPT]) {
+        float* dst = a.out + ((size_t)(s0 + tt) * a.H + h) * dv + col;
+        if (MODE == PRISM_SCAN_TOKEN)
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) o[p] += skip * f1[NV * dkp + lc + p];
+        if (CPT == 4) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1 % CPT], o[2 % CPT], o[3 % CPT]);
+        else if (CPT == 2) *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1 % CPT]);
+        else dst[0] = o[0];
+    };
+
     int buf = 0;
     for (int b0 = 0; b0 < qlen; b0 += TB, buf = buf + 1 == NBUF ? 0 : buf + 1) {
         const int nb = min(TB, qlen - b0);
         if (producer) {
-            // while block b0 is worked on: ask for the block after the next (its buffer was freed at the last
-            // barrier), and see the next one in
-            const int nxt = buf + 1 == NBUF ? 0 : buf + 1, nxt2 = nxt + 1 == NBUF ? 0 : nxt + 1;
-            if (b0 + 2 * TB < qlen) stage(b0 + 2 * TB, nxt2);
+            // while block b0 is worked on: ask for the block that goes into the buffer freed at the last barrier, and
+            // see the next one in
+            const int nxt = buf + 1 == NBUF ? 0 : buf + 1, freed = buf == 0 ? NBUF - 1 : buf - 1;
+            if (b0 + (NBUF - 1) * TB < qlen) stage(b0 + (NBUF - 1) * TB, freed);
             else cp_async_commit();
-            cp_async_wait<1>();
+            cp_async_wait_upto(NBUF - 2);
             if (b0 + TB < qlen) finish(b0 + TB, nxt);
             __syncthreads();
             continue;
         }
         const float* blk = sm + (size_t)buf * TB * per_tok;
-        for (int tt = 0; tt < nb; ++tt) {
-            const float* f1 = blk + (size_t)tt * per_tok;          // q or r
-            const float* f2 = f1 + dkp;                            // k
-            float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;         // four chains of multiply-adds side by side
-            if (MODE == PRISM_SCAN_DELTA) {
-                const float* vv = f2 + dkp;
-                const float beta = vv[a.colsp], g = vv[a.colsp + 1];
-                float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
-                float4 kq[Q];
+        int tt = 0;
+        if constexpr (LONG) {                          // L is 8
+            for (; tt + 8 <= nb; tt += 8) {
+                float o[8][CPT];
+                ulonglong2 q[2][Q];
 #pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    kq[m] = *reinterpret_cast<const float4*>(f2 + 4 * (part + L * m));
-                    k0 += S[4 * m] * kq[m].x;
-                    k1 += S[4 * m + 1] * kq[m].y;
-                    k2 += S[4 * m + 2] * kq[m].z;
-                    k3 += S[4 * m + 3] * kq[m].w;
-                }
-                float ks = (k0 + k1) + (k2 + k3);
-                ks = column_sum<L>(ks);
-                const float uu = beta * (vv[lc] - g * ks);
+                for (int i = 0; i < 8; ++i)
+                    token(blk + (size_t)(tt + i) * per_tok, q[i & 1], o[i], i > 0, q[(i + 1) & 1], o[(i + 7) & 7]);
+                read(q[1], o[7]);
+                // the eight tokens' sums over the eight lanes of a column, each lane ends with one token's: the same
+                // pairs as column_sum's, half of the values a level
+                float r[CPT];
 #pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const float4 qq = *reinterpret_cast<const float4*>(f1 + 4 * (part + L * m));
-                    S[4 * m] = g * S[4 * m] + kq[m].x * uu;
-                    S[4 * m + 1] = g * S[4 * m + 1] + kq[m].y * uu;
-                    S[4 * m + 2] = g * S[4 * m + 2] + kq[m].z * uu;
-                    S[4 * m + 3] = g * S[4 * m + 3] + kq[m].w * uu;
-                    o0 += S[4 * m] * qq.x;
-                    o1 += S[4 * m + 1] * qq.y;
-                    o2 += S[4 * m + 2] * qq.z;
-                    o3 += S[4 * m + 3] * qq.w;
-                }
-            } else if (MODE == PRISM_SCAN_CHANNEL) {
-                const float* wd = f2 + dkp;
-                const float* vv = wd + dkp;
-                const float beta = vv[a.colsp];
-                float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
-                float4 kq[Q];
+                for (int p = 0; p < CPT; ++p) {
+                    float h4[4], h2[2];
 #pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const int i = 4 * (part + L * m);
-                    kq[m] = *reinterpret_cast<const float4*>(f2 + i);
-                    const float4 w4 = *reinterpret_cast<const float4*>(wd + i);
-                    S[4 * m] *= w4.x;
-                    S[4 * m + 1] *= w4.y;
-                    S[4 * m + 2] *= w4.z;
-                    S[4 * m + 3] *= w4.w;
-                    k0 += S[4 * m] * kq[m].x;
-                    k1 += S[4 * m + 1] * kq[m].y;
-                    k2 += S[4 * m + 2] * kq[m].z;
-                    k3 += S[4 * m + 3] * kq[m].w;
-                }
-                float ks = (k0 + k1) + (k2 + k3);
-                ks = column_sum<L>(ks);
-                const float uu = beta * (vv[lc] - ks);
+                    for (int i = 0; i < 4; ++i) {
+                        const float mine = part & 4 ? o[i + 4][p] : o[i][p], other = part & 4 ? o[i][p] : o[i + 4][p];
+                        h4[i] = mine + __shfl_xor_sync(0xffffffffu, other, 4);
+                    }
 #pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const float4 qq = *reinterpret_cast<const float4*>(f1 + 4 * (part + L * m));
-                    S[4 * m] += kq[m].x * uu;
-                    S[4 * m + 1] += kq[m].y * uu;
-                    S[4 * m + 2] += kq[m].z * uu;
-                    S[4 * m + 3] += kq[m].w * uu;
-                    o0 += S[4 * m] * qq.x;
-                    o1 += S[4 * m + 1] * qq.y;
-                    o2 += S[4 * m + 2] * qq.z;
-                    o3 += S[4 * m + 3] * qq.w;
+                    for (int i = 0; i < 2; ++i) {
+                        const float mine = part & 2 ? h4[i + 2] : h4[i], other = part & 2 ? h4[i] : h4[i + 2];
+                        h2[i] = mine + __shfl_xor_sync(0xffffffffu, other, 2);
+                    }
+                    const float mine = part & 1 ? h2[1] : h2[0], other = part & 1 ? h2[0] : h2[1];
+                    r[p] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
                 }
-            } else if (MODE == PRISM_SCAN_GENERAL) {
-                const float* wd = f2 + dkp;            // decay | unit key | removal times unit key | v
-                const float* ue = wd + dkp;
-                const float* ce = ue + dkp;
-                const float v = ce[dkp + lc];
-                float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
-#pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const float4 e4 = *reinterpret_cast<const float4*>(ue + 4 * (part + L * m));
-                    k0 += S[4 * m] * e4.x;
-                    k1 += S[4 * m + 1] * e4.y;
-                    k2 += S[4 * m + 2] * e4.z;
-                    k3 += S[4 * m + 3] * e4.w;
-                }
-                float es = (k0 + k1) + (k2 + k3);
-                es = column_sum<L>(es);                // e^T S of this column, from the state before the token
-#pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const int i = 4 * (part + L * m);
-                    const float4 rr = *reinterpret_cast<const float4*>(f1 + i), kk = *reinterpret_cast<const float4*>(f2 + i);
-                    const float4 w4 = *reinterpret_cast<const float4*>(wd + i), c4 = *reinterpret_cast<const float4*>(ce + i);
-                    S[4 * m] = w4.x * S[4 * m] - c4.x * es + kk.x * v;
-                    S[4 * m + 1] = w4.y * S[4 * m + 1] - c4.y * es + kk.y * v;
-                    S[4 * m + 2] = w4.z * S[4 * m + 2] - c4.z * es + kk.z * v;
-                    S[4 * m + 3] = w4.w * S[4 * m + 3] - c4.w * es + kk.w * v;
-                    o0 += S[4 * m] * rr.x;
-                    o1 += S[4 * m + 1] * rr.y;
-                    o2 += S[4 * m + 2] * rr.z;
-                    o3 += S[4 * m + 3] * rr.w;
-                }
-            } else if (MODE == PRISM_SCAN_RETAIN || MODE == PRISM_SCAN_TOKEN) {
-                const float* vv = f2 + dkp;
-                const float g = MODE == PRISM_SCAN_TOKEN ? vv[a.colsp + 1] : keep;
-                const float v = MODE == PRISM_SCAN_TOKEN ? vv[a.colsp] * vv[lc] : vv[lc];
-#pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const int i = 4 * (part + L * m);
-                    const float4 qq = *reinterpret_cast<const float4*>(f1 + i), kk = *reinterpret_cast<const float4*>(f2 + i);
-                    S[4 * m] = g * S[4 * m] + kk.x * v;
-                    S[4 * m + 1] = g * S[4 * m + 1] + kk.y * v;
-                    S[4 * m + 2] = g * S[4 * m + 2] + kk.z * v;
-                    S[4 * m + 3] = g * S[4 * m + 3] + kk.w * v;
-                    o0 += S[4 * m] * qq.x;
-                    o1 += S[4 * m + 1] * qq.y;
-                    o2 += S[4 * m + 2] * qq.z;
-                    o3 += S[4 * m + 3] * qq.w;
-                }
-            } else if (MODE == PRISM_SCAN_GATED) {
-                const float* wd = f2 + dkp;
-                const float v = wd[dkp + lc];
-#pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const int i = 4 * (part + L * m);
-                    const float4 qq = *reinterpret_cast<const float4*>(f1 + i), kk = *reinterpret_cast<const float4*>(f2 + i);
-                    const float4 w4 = *reinterpret_cast<const float4*>(wd + i);
-                    S[4 * m] = w4.x * S[4 * m] + kk.x * v;
-                    S[4 * m + 1] = w4.y * S[4 * m + 1] + kk.y * v;
-                    S[4 * m + 2] = w4.z * S[4 * m + 2] + kk.z * v;
-                    S[4 * m + 3] = w4.w * S[4 * m + 3] + kk.w * v;
-                    o0 += S[4 * m] * qq.x;
-                    o1 += S[4 * m + 1] * qq.y;
-                    o2 += S[4 * m + 2] * qq.z;
-                    o3 += S[4 * m + 3] * qq.w;
-                }
-            } else {
-                const float* wd = f2 + dkp;
-                const float v = wd[dkp + lc];
-#pragma unroll
-                for (int m = 0; m < Q; ++m) {
-                    const int i = 4 * (part + L * m);
-                    const float4 rr = *reinterpret_cast<const float4*>(f1 + i), kk = *reinterpret_cast<const float4*>(f2 + i);
-                    const float4 w4 = *reinterpret_cast<const float4*>(wd + i), u4 = *reinterpret_cast<const float4*>(ub + i);
-                    const float kv0 = kk.x * v, kv1 = kk.y * v, kv2 = kk.z * v, kv3 = kk.w * v;
-                    o0 += rr.x * (S[4 * m] + u4.x * kv0);
-                    o1 += rr.y * (S[4 * m + 1] + u4.y * kv1);
-                    o2 += rr.z * (S[4 * m + 2] + u4.z * kv2);
-                    o3 += rr.w * (S[4 * m + 3] + u4.w * kv3);
-                    S[4 * m] = w4.x * S[4 * m] + kv0;
-                    S[4 * m + 1] = w4.y * S[4 * m + 1] + kv1;
-                    S[4 * m + 2] = w4.z * S[4 * m + 2] + kv2;
-                    S[4 * m + 3] = w4.w * S[4 * m + 3] + kv3;
-                }
+                if (live) store(b0 + tt + part, blk + (size_t)(tt + part) * per_tok, r);
             }
-            float o = (o0 + o1) + (o2 + o3);
-            o = column_sum<L>(o);
-            if (MODE == PRISM_SCAN_TOKEN) o += skip * f2[dkp + lc];
-            if (live && part == 0) a.out[((size_t)(s0 + b0 + tt) * a.H + h) * dv + col] = o;
+        }
+        for (; tt < nb; ++tt) {
+            float o[CPT];
+            ulonglong2 q[Q];
+            token(blk + (size_t)tt * per_tok, q, o, false, q, o);
+            read(q, o);
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) o[p] = column_sum<L>(o[p]);
+            if (live && part == 0) store(b0 + tt, blk + (size_t)tt * per_tok, o);
         }
         __syncthreads();                               // the next block has landed, and this buffer is free
     }
@@ -700,26 +813,33 @@ __global__ void scan_kernel(const ScanArgs a) {
 #pragma unroll
         for (int m = 0; m < Q; ++m) {
             const int i = 4 * (part + L * m);
-            if (a.vec && i + 3 < dk) {
-                *reinterpret_cast<float4*>(st + i) = make_float4(S[4 * m], S[4 * m + 1], S[4 * m + 2], S[4 * m + 3]);
-            } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (i + j < dk) st[i + j] = S[4 * m + j];
+            for (int p = 0; p < CPT; ++p) {
+                float* sp = st + (size_t)p * dk + i;
+                const float2 lo = unpack2(S[p][2 * m]), hi = unpack2(S[p][2 * m + 1]);
+                if (a.vec && i + 3 < dk) {
+                    *reinterpret_cast<float4*>(sp) = make_float4(lo.x, lo.y, hi.x, hi.y);
+                } else {
+                    const float v[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (i + j < dk) sp[j] = v[j];
+                }
             }
         }
     }
 }
 
-template <int MODE, int R, int L>
+template <int MODE, int R, int L, int CPT = 1, bool LONG = false>
 static int launch_scan(const ScanArgs& a, int S, cudaStream_t stream) {
     const int per_tok = scan_vectors(MODE) * a.dkp + a.colsp + 4;
-    const size_t smem = ((size_t)3 * a.TB * per_tok + (MODE == PRISM_SCAN_BONUS ? a.dkp : 0)) * sizeof(float);
-    auto kern = scan_kernel<MODE, R, L>;
+    const size_t smem = (size_t)a.NBUF * a.TB * per_tok * sizeof(float);
+    static_assert(!LONG || L == 8, "");
+    auto kern = scan_kernel<MODE, R, L, CPT, LONG>;
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid(a.H, S, (a.dv + a.cols - 1) / a.cols);
-    return (int)launch_kernel(kern, grid, dim3((a.cols * a.L + 31) / 32 * 32 + 32), smem, stream, a);      // + the producer warp
+    return (int)launch_kernel(kern, grid, dim3((a.cols / CPT * a.L + 31) / 32 * 32 + 32), smem, stream, a);      // + the producer warp
 }
 
 }  // namespace prism
@@ -872,37 +992,60 @@ PRISM_EXPORT int prism_recurrent_scan(int mode, const float* x, long long x_stri
     if (mode == PRISM_SCAN_RETAIN && (w0 == nullptr || rep != 1)) return (int)cudaErrorInvalidValue;
     if (mode == PRISM_SCAN_GENERAL && (ex == nullptr || ww == nullptr || rep != 1)) return (int)cudaErrorInvalidValue;
     if ((mode == PRISM_SCAN_TOKEN && bg == nullptr) || (mode == PRISM_SCAN_GATED && (ww == nullptr || rep != 1))) return (int)cudaErrorInvalidValue;
-    // A token's work is one chain (dot product, shuffles, update, dot product, shuffles), so a CTA is latency
-    // bound: eight threads a column, four warps of them side by side, and as many CTAs as there are column blocks.
     const int R = dk <= 32 ? 4 : (dk <= 64 ? 8 : (dk <= 128 ? 16 : 32));
     int L = 1;
     while (L * R < dk) L *= 2;                          // at most 32
     if (R >= 8 && L < 8) L = 8;                        // the compiled pairs: more than 32 rows always take eight threads a column
     a.L = L;
     a.dkp = L * R;                                     // the rows the threads of a column cover; beyond dk: zeros
-    // 128 threads a CTA beside the producer warp; fewer (down to one warp) while the grid would leave SMs idle
-    int threads = 128;
-    while (threads > 32 && (long long)H * S * ((dv + threads / L - 1) / (threads / L)) < 148) threads /= 2;
-    int cols = threads / L < 1 ? 1 : threads / L;
+    const bool quads = dk % 4 == 0 && dv % 4 == 0 && x_stride % 4 == 0 && qo % 4 == 0 && ko % 4 == 0 && vo % 4 == 0 &&
+                       (uintptr_t)x % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0 &&
+                       (scan_vectors(mode) == 2 || (ww_stride % 4 == 0 && (uintptr_t)ww % 16 == 0)) &&
+                       (mode != PRISM_SCAN_GENERAL || (ex_stride % 4 == 0 && (uintptr_t)ex % 16 == 0 && ((long long)H * dk) % 4 == 0));
+    // Columns a CTA: the fewest of 4 to 64 whose CTAs fit the 148 SMs once, since a second CTA on an SM shares its
+    // schedulers and shared memory while the chain of tokens takes as long (2,048 tokens, delta rule, 16 heads of 128:
+    // 16 columns 296 us, 8 columns on two CTAs an SM 346 us; 32 heads: 32 columns 370 us, 16 columns 587 us).  More than
+    // 4 x 4 of them give a thread several, so that the token's vectors are read fewer times.  The modes with three
+    // vectors and more do better where each warp has twice the columns a thread and a CTA of its own (2,048 columns,
+    // general, 1,024 tokens: 212 us, 16 columns as four warps 230 us; bonus, 2,048 tokens: 178 and 255 us), the others
+    // not (delta: 330 and 296 us).  A few tokens a request are bound by the state's way in and out: one column a thread.
+    int cpt = 1, threads = 128;
+    auto ctas = [&](int cols) { return (long long)H * S * ((dv + cols - 1) / cols); };
+    const bool many = quads && L == 8 && (R == 8 || R == 16) && max_q_len >= 16;
+    if (many) {
+        int want = 4;
+        while (want < 64 && ctas(want) > 148) want *= 2;
+        cpt = want <= 16 ? 1 : (want == 32 ? 2 : 4);
+        if (scan_vectors(mode) > 2 && (want == 16 || want == 32)) cpt *= 2, want /= 2;
+        threads = want / cpt * L;
+    } else {
+        while (threads > 32 && ctas(threads / L) < 148) threads /= 2;
+    }
+    int cols = threads / L < 1 ? 1 : threads / L * cpt;
     if (cols > dv) cols = dv;
     if (cols >= 4) cols = cols / 4 * 4;
     a.cols = cols;
     a.colsp = (cols + 3) / 4 * 4;
-    a.vec = dk % 4 == 0 && dv % 4 == 0 && cols % 4 == 0 && x_stride % 4 == 0 && qo % 4 == 0 && ko % 4 == 0 && vo % 4 == 0 &&
-            (uintptr_t)x % 16 == 0 && (uintptr_t)state % 16 == 0 &&
-            (scan_vectors(mode) == 2 || (ww_stride % 4 == 0 && (uintptr_t)ww % 16 == 0)) &&
-            (mode != PRISM_SCAN_GENERAL || (ex_stride % 4 == 0 && (uintptr_t)ex % 16 == 0 && ((long long)H * dk) % 4 == 0));
+    a.vec = quads && cols % 4 == 0;
     const int per_tok = scan_vectors(mode) * a.dkp + a.colsp + 4;
     int tb = (24 * 1024 / 4) / per_tok;
-    tb = tb < 1 ? 1 : (tb > 16 ? 16 : tb);
+    tb = tb < 1 ? 1 : (tb >= 16 ? 16 : (tb >= 8 ? 8 : tb));
     a.TB = tb > max_q_len ? (max_q_len < 1 ? 1 : max_q_len) : tb;      // a decode step stages one token, and CTAs are small
+    // blocks on their way cover the latency of memory at some 100 ns a token; 100 KB leave room for two CTAs an SM
+    const int blocks = (max_q_len + a.TB - 1) / a.TB;
+    a.NBUF = 100 * 1024 / (a.TB * per_tok * 4);
+    a.NBUF = a.NBUF > 8 ? 8 : a.NBUF;
+    if (a.NBUF > blocks + 1) a.NBUF = blocks + 1;
+    if (a.NBUF < 3) a.NBUF = 3;
     // rows a thread and threads a column, both known to the compiler: (4, 1..8) up to 32 rows, (8, 8), (16, 8), (32, 8..32)
 #define PRISM_SCAN(M)                                                                                \
     do {                                                                                             \
         if (R == 4) return L == 1 ? launch_scan<M, 4, 1>(a, S, stream) : L == 2 ? launch_scan<M, 4, 2>(a, S, stream)    \
                          : L == 4 ? launch_scan<M, 4, 4>(a, S, stream) : launch_scan<M, 4, 8>(a, S, stream);           \
-        if (R == 8) return launch_scan<M, 8, 8>(a, S, stream);                                       \
-        if (R == 16) return launch_scan<M, 16, 8>(a, S, stream);                                     \
+        if (R == 8) return cpt == 4 ? launch_scan<M, 8, 8, 4, true>(a, S, stream) : cpt == 2 ? launch_scan<M, 8, 8, 2, true>(a, S, stream) \
+                         : many ? launch_scan<M, 8, 8, 1, true>(a, S, stream) : launch_scan<M, 8, 8>(a, S, stream);                                       \
+        if (R == 16) return cpt == 4 ? launch_scan<M, 16, 8, 4, true>(a, S, stream) : cpt == 2 ? launch_scan<M, 16, 8, 2, true>(a, S, stream) \
+                         : many ? launch_scan<M, 16, 8, 1, true>(a, S, stream) : launch_scan<M, 16, 8>(a, S, stream);                                      \
         return L == 8 ? launch_scan<M, 32, 8>(a, S, stream) : L == 16 ? launch_scan<M, 32, 16>(a, S, stream)           \
                       : launch_scan<M, 32, 32>(a, S, stream);                                        \
     } while (0)

@@ -864,3 +864,87 @@ def test_attention_window_edge(kind):
                 assert torch.allclose(last, torch.full_like(last, 7.0), atol=0.05), (kind, ctx, "inside key not found")
             else:
                 assert float(last.abs().max()) < 3.0, (kind, ctx, "key outside the window was seen", float(last.abs().max()))
+
+
+def _scan_reference(mode, q, k, v, w, u, e, c, beta, g):
+    """The recurrences of csrc/recurrent.cu for one request, all heads at once, float64: rows ``[T, H, .]``."""
+    T, H, d = q.shape
+    S = torch.zeros(H, d, v.shape[-1], dtype=torch.float64, device=q.device)
+    out = []
+    outer = lambda a, b: a[:, :, None] * b[:, None, :]                                     # noqa: E731
+    for t in range(T):
+        dot = lambda a: (S * a[:, :, None]).sum(1)                                         # noqa: E731
+        if mode in ("delta", "channel"):
+            S = S * (g[t][:, None, None] if mode == "delta" else w[t][:, :, None])
+            S = S + outer(k[t], beta[t][:, None] * (v[t] - dot(k[t])))
+        elif mode == "general":
+            S = w[t][:, :, None] * S - outer(c[t], dot(e[t])) + outer(k[t], v[t])
+        elif mode == "bonus":
+            now = S + outer(u * k[t], v[t])
+            out.append((now * q[t][:, :, None]).sum(1))
+            S = w[t][:, :, None] * S + outer(k[t], v[t])
+            continue
+        elif mode == "token":
+            S = g[t][:, None, None] * S + outer(k[t], beta[t][:, None] * v[t])
+        else:
+            S = (w[t] if mode == "gated" else u[:, :1].expand_as(w[t]))[:, :, None] * S + outer(k[t], v[t])
+        out.append(dot(q[t]) + (u[:, :1] * v[t] if mode == "token" else 0))
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("mode", ["delta", "bonus", "channel", "general", "retain", "token", "gated"])
+@pytest.mark.parametrize("H,dk,dv,lens", [(3, 64, 64, (37,)), (16, 128, 64, (17, 40)), (9, 100, 100, (33, 9, 16)), (16, 64, 128, (24, 3, 41))])
+def test_scan_at_every_split(mode, H, dk, dv, lens):
+    """Requests whose columns a CTA takes 8 (few heads) to 64 at a time, one to four a thread, in remainders of the
+    blocks of eight tokens: against the recurrence in float64, and bit for bit the same when cut into single tokens
+    and portions.  Bound: rounding 2^-24 of values of about 1, at most T additions deep and dk + 8 wide a token."""
+    from types import SimpleNamespace
+    ops = _ops()
+    gen = torch.Generator().manual_seed(dk + H)
+    T, A, B = sum(lens), H * dk, H * dv
+    n = lambda *s: torch.randn(*s, generator=gen)                                         # noqa: E731
+    unit = lambda x: torch.nn.functional.normalize(x, dim=-1)                             # noqa: E731
+    q, k, v = unit(n(T, H, dk)), unit(n(T, H, dk)), n(T, H, dv)
+    w = 0.9 + 0.1 * torch.rand(T, H, dk, generator=gen)
+    e, u = unit(n(T, H, dk)), n(H, dk)
+    c = e * torch.rand(T, H, dk, generator=gen)
+    beta, g = torch.rand(T, H, generator=gen), 0.9 + 0.1 * torch.rand(T, H, generator=gen)
+    if mode in ("retain", "token"):
+        u[:, :] = 0.9 + 0.1 * torch.rand(H, 1, generator=gen)
+    x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(DEV)
+    kw = {"delta": dict(bg=torch.cat([beta, g], 1)), "token": dict(bg=torch.cat([beta, g], 1), w0=u[:, 0]),
+          "bonus": dict(ww=w.reshape(T, A), w0=torch.zeros(A), u=u.reshape(A), decay_ready=True),
+          "channel": dict(bg=beta, ww=w.reshape(T, A)), "gated": dict(ww=w.reshape(T, A)), "retain": dict(w0=u[:, 0]),
+          "general": dict(ww=w.reshape(T, A), ex=torch.cat([e.reshape(T, A), c.reshape(T, A)], 1))}[mode]
+    kw = {a: b if isinstance(b, bool) else b.contiguous().to(DEV) for a, b in kw.items()}
+    code = dict(delta=ops.SCAN_DELTA, bonus=ops.SCAN_BONUS, channel=ops.SCAN_CHANNEL, general=ops.SCAN_GENERAL,
+                retain=ops.SCAN_RETAIN, token=ops.SCAN_TOKEN, gated=ops.SCAN_GATED)[mode]
+
+    def go(parts):                           # parts: (request, first row, rows) of a step, one after another
+        rows = torch.cat([torch.arange(a, a + m) for _, a, m in parts]).to(DEV)
+        start = torch.tensor([0] + [m for _, _, m in parts]).cumsum(0).to(torch.int32).to(DEV)
+        ctx = SimpleNamespace(seg_start=start, S=len(parts), max_q_len=max(m for _, _, m in parts),
+                              state_slots=torch.tensor([r for r, _, _ in parts], dtype=torch.int32, device=DEV))
+        xs, out = x[rows], torch.empty(len(rows), H, dv, device=DEV)
+        some = {a: b[rows] if torch.is_tensor(b) and a in ("bg", "ww", "ex") else b for a, b in kw.items()}
+        ops.recurrent_scan(code, xs[:, :A], xs[:, A:2 * A], xs[:, 2 * A:], state, ctx, H, 1, dk, dv, out, **some)
+        return rows, out
+
+    first = [sum(lens[:i]) for i in range(len(lens))]
+    state = torch.zeros(len(lens), H, dv, dk, device=DEV)
+    _, whole = go([(i, first[i], m) for i, m in enumerate(lens)])
+    kept, state = state, torch.zeros_like(state)
+    cut, at = torch.empty_like(whole), [0] * len(lens)
+    for size in (1, 17, 2, 9, 1, 64):
+        parts = [(i, first[i] + at[i], min(size, m - at[i])) for i, m in enumerate(lens) if at[i] < m]
+        if parts:
+            rows, out = go(parts)
+            cut[rows] = out
+            at = [min(a + size, m) for a, m in zip(at, lens)]
+    assert torch.equal(whole, cut) and torch.equal(kept, state)
+    for i, m in enumerate(lens):
+        s = slice(first[i], first[i] + m)
+        d = [t.double().to(DEV) for t in (q[s], k[s], v[s], w[s], u, e[s], c[s], beta[s], g[s])]
+        ref = _scan_reference(mode, *d)
+        bound = 2.0 ** -24 * (m + dk + 8) * max(1.0, float(ref.abs().max()))
+        assert float((whole[s].double() - ref).abs().max()) <= bound, (i, bound)
