@@ -482,6 +482,27 @@ def test_attention_generic(case, dtype):
     assert torch.allclose(out.float(), ref, atol=tol, rtol=tol)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window,segs", [
+    (14, 2, 64, None, [(0, 90), (300, 1), (31, 2)]), (6, 1, 128, 70, [(0, 200)]), (9, 3, 40, None, [(513, 1), (0, 120)]),
+    (3, 3, 100, None, [(290, 2), (0, 70)])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_in_one_order(nh, nkv, hd, window, segs, dtype):
+    """Several heads of a kv head a CTA, or one, with remainders of heads, blocks, rows and warps: against the reference,
+    and bit for bit what a token gives alone."""
+    ops = _ops()
+    c = PagedCase(segs, nh, nkv, hd, 16, dtype, seed=21)
+    out, err, scale = torch.empty(c.T, nh * hd, dtype=dtype, device=DEV), _err(), hd ** -0.5
+    ops.attention_generic(c.q, out, c.k, c.v, c.bt, c.positions, c.tok_seg, c.num_pages, window, scale, err)
+    ref = ref_paged_attention(c.q, c.k, c.v, c.bt, c.positions, c.tok_seg, window, scale)
+    tol = 2e-5 if dtype == torch.float32 else 2e-2
+    assert int(err) == 0 and torch.allclose(out.float(), ref, atol=tol, rtol=tol)
+    for t in (0, 1, 31, 32, 63, c.T - 2, c.T - 1):
+        one = torch.empty(1, nh * hd, dtype=dtype, device=DEV)
+        ops.attention_generic(c.q[t:t + 1], one, c.k, c.v, c.bt, c.positions[t:t + 1], c.tok_seg[t:t + 1], c.num_pages, window,
+                              scale, err)
+        assert torch.equal(one[0], out[t]), t
+
+
 def test_attention_generic_rejects_big_head():
     ops = _ops()
     c = PagedCase([(0, 2)], 1, 1, 272, 16, torch.float32, seed=1)
