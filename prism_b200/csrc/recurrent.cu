@@ -111,6 +111,96 @@ __global__ void conv_unit_gates_kernel(const float* __restrict__ proj_in, long l
     }
 }
 
+// The same for a step of many tokens: a warp takes one head's channels (q, k or v; d = lane + 32 m) of RUN tokens one
+// after another with the inputs of the last K - 1 tokens and the taps in registers, so that every input is read once
+// instead of K times and nothing passes through shared memory; sums in the order of the kernel above.  One more "head"
+// forms the gates.  Bound by the bytes of proj and qkv: 2,048 tokens of 6,144 channels 78 us by the kernel above,
+// 13 us here.
+constexpr int CONV_RUN = 16, CONV_TAPS = 4;
+template <int M>
+__global__ void __launch_bounds__(128) conv_unit_gates_run_kernel(const float* __restrict__ proj_in, long long ps, int ob, int oa,
+                                                                  const void* __restrict__ taps, int taps_bf16, int K,
+                                                                  const float* tail, const void* __restrict__ a_log, int a_log_bf16,
+                                                                  const void* __restrict__ dt_bias, int dt_bf16,
+                                                                  const int* __restrict__ tok_seg, const int* __restrict__ seg_start,
+                                                                  const int* __restrict__ slots, int T, int G, int H, int dk, int dv,
+                                                                  float unit_eps, float* __restrict__ qkv, float* __restrict__ bg) {
+    pdl_trigger();
+    pdl_wait();
+    const float* proj = pdl_fresh(proj_in);
+    const int lane = threadIdx.x & 31, hh = blockIdx.y * 4 + (threadIdx.x >> 5);       // neighbouring warps: neighbouring channels
+    const int t0 = blockIdx.x * CONV_RUN, t1 = min(T, t0 + CONV_RUN);
+    const int C = 2 * G * dk + H * dv;
+    if (hh > 2 * G + H) return;
+    if (hh == 2 * G + H) {
+        for (int i = lane; i < (t1 - t0) * H; i += 32) {
+            const int t = t0 + i / H, h = i % H;
+            const float beta = sigmoid_f(proj[(size_t)t * ps + ob + h]);
+            if (a_log == nullptr) {
+                bg[(size_t)t * H + h] = beta;
+            } else {
+                bg[(size_t)t * 2 * H + h] = beta;
+                const float dt = softplus_f(proj[(size_t)t * ps + oa + h] + load_param(dt_bias, dt_bf16, h));
+                bg[(size_t)t * 2 * H + H + h] = expf(-expf(load_param(a_log, a_log_bf16, h)) * dt);
+            }
+        }
+        return;
+    }
+    const bool unit = hh < 2 * G;
+    const int n = unit ? dk : dv, c0 = unit ? hh * dk : 2 * G * dk + (hh - 2 * G) * dv;
+    float w[CONV_TAPS][M], x[CONV_TAPS][M];            // lag j: tap and input of j tokens back (lags from K on: zero)
+#pragma unroll
+    for (int j = 0; j < CONV_TAPS; ++j)
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int d = lane + 32 * m;
+            w[j][m] = j < K && d < n ? load_param(taps, taps_bf16, (size_t)(c0 + d) * K + (K - 1 - j)) : 0.f;
+            x[j][m] = 0.f;
+        }
+    int seg = -1, s0 = 0, s1 = 0;
+    float ahead[M];                                    // the next token's inputs, asked for before this one's are used
+#pragma unroll
+    for (int m = 0; m < M; ++m) ahead[m] = lane + 32 * m < n ? proj[(size_t)t0 * ps + c0 + lane + 32 * m] : 0.f;
+    for (int t = t0; t < t1; ++t) {
+        if (t >= s1) {                                 // the run's first token, or a segment's: the inputs before it
+            seg = tok_seg[t], s0 = seg_start[seg], s1 = seg_start[seg + 1];
+            const float* tl = tail + (size_t)slots[seg] * (K - 1) * C;
+#pragma unroll
+            for (int j = 0; j + 1 < CONV_TAPS; ++j) {  // becomes lag j + 1
+                const int src = t - s0 - 1 - j;
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int d = lane + 32 * m;
+                    x[j][m] = j + 1 < K && d < n ? (src >= 0 ? proj[(size_t)(t - 1 - j) * ps + c0 + d] : tl[(size_t)(K - 1 + src) * C + c0 + d]) : 0.f;
+                }
+            }
+        }
+        float y[M], ss = 0.f;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+#pragma unroll
+            for (int j = CONV_TAPS - 1; j > 0; --j) x[j][m] = x[j - 1][m];
+            x[0][m] = ahead[m];
+            if (t + 1 < t1) ahead[m] = lane + 32 * m < n ? proj[(size_t)(t + 1) * ps + c0 + lane + 32 * m] : 0.f;
+            float acc = 0.f;
+#pragma unroll
+            for (int j = CONV_TAPS - 1; j >= 0; --j)
+                if (j < K) acc += w[j][m] * x[j][m];
+            y[m] = silu_f(acc);
+            if (lane + 32 * m < n) ss += y[m] * y[m];
+        }
+        if (unit) {
+            ss = warp_sum(ss);
+            const float inv = (1.f / sqrtf(ss + unit_eps)) * (hh < G ? 1.f / sqrtf((float)dk) : 1.f);
+#pragma unroll
+            for (int m = 0; m < M; ++m) y[m] *= inv;
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            if (lane + 32 * m < n) qkv[(size_t)t * C + c0 + lane + 32 * m] = y[m];
+    }
+}
+
 // tail[slot][r][c] <- the input (rows - r) tokens before the end of the request's tokens so far: from this
 // step's rows where the step reaches that far back, else from the tail as it was (shifted).  One CTA per
 // segment; a thread owns a column, and walks r upwards, so that what it still needs is never overwritten.
@@ -259,16 +349,31 @@ __global__ void headnorm_gate_kernel(const float* __restrict__ o_in, const float
     if (w >= (long long)Ttot * H) return;
     const int t = (int)(w / H), h = (int)(w % H);
     const float* row = o + ((size_t)t * H + h) * dv;
+    const float* gr = gate + (size_t)t * gs + (size_t)h * dv;
+    constexpr int AHEAD = 4;                           // entries a lane keeps: rows and gates of up to 128 are all on their way
+                                                       // before the sum (2,048 tokens, 16 heads of 128: 26 -> 19 us)
+    float x[AHEAD], g4[AHEAD];
     float ss = 0.f;
-    for (int c = lane; c < dv; c += 32) ss += row[c] * row[c];
+#pragma unroll
+    for (int m = 0; m < AHEAD; ++m) {
+        const int c = lane + 32 * m;
+        x[m] = c < dv ? row[c] : 0.f;
+        g4[m] = c < dv ? gr[c] : 0.f;
+    }
+#pragma unroll
+    for (int m = 0; m < AHEAD; ++m) ss += x[m] * x[m];
+    for (int c = lane + 32 * AHEAD; c < dv; c += 32) ss += row[c] * row[c];
     ss = warp_sum(ss);
     const float inv = 1.f / sqrtf(ss / (float)dv + eps);
-    for (int c = lane; c < dv; c += 32) {
+    auto put = [&](int c, float v, float gz) {
         const float wv = weight != nullptr ? load_param(weight, weight_bf16, per_head_weight ? (size_t)h * dv + c : (size_t)c) : 1.f;
-        const float gz = gate[(size_t)t * gs + (size_t)h * dv + c];
         const float g = gate_sigmoid == 2 ? gz : (gate_sigmoid ? sigmoid_f(gz) : silu_f(gz));
-        out[(size_t)t * os + (size_t)h * dv + c] = from_float<T>(row[c] * inv * wv * g * scale);
-    }
+        out[(size_t)t * os + (size_t)h * dv + c] = from_float<T>(v * inv * wv * g * scale);
+    };
+#pragma unroll
+    for (int m = 0; m < AHEAD; ++m)
+        if (lane + 32 * m < dv) put(lane + 32 * m, x[m], g4[m]);
+    for (int c = lane + 32 * AHEAD; c < dv; c += 32) put(c, row[c], gr[c]);
 }
 
 // bg[t][h] = softplus(z[t][h] + bias[h]) (a step size) and bg[t][H + h] = exp(-exp(a_log[h]) times it) (the decay it makes).
@@ -854,6 +959,18 @@ PRISM_EXPORT int prism_conv_unit_gates(const float* proj, long long ps, int ob, 
     const int C = 2 * G * dk + H * dv;
     const size_t smem = (size_t)C * sizeof(float);
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
+    // runs of tokens where there are enough of them to fill the GPU with a warp a head and run
+    const int widest = dk > dv ? dk : dv;
+    if (!move_tail && K <= prism::CONV_TAPS && widest <= 128 && T >= 256) {
+        const dim3 grid((T + prism::CONV_RUN - 1) / prism::CONV_RUN, (2 * G + H + 1 + 3) / 4);
+        auto run = [&](auto kernel) {
+            return (int)prism::launch_kernel(kernel, grid, dim3(128), 0, stream, proj, ps, ob, oa, taps, taps_dtype == PRISM_DTYPE_BF16, K,
+                                             tail, a_log, a_log_dtype == PRISM_DTYPE_BF16, dt_bias, dt_dtype == PRISM_DTYPE_BF16, tok_seg,
+                                             seg_start, slots, T, G, H, dk, dv, unit_eps, qkv, bg);
+        };
+        return widest <= 32 ? run(prism::conv_unit_gates_run_kernel<1>) : widest <= 64 ? run(prism::conv_unit_gates_run_kernel<2>)
+                            : run(prism::conv_unit_gates_run_kernel<4>);
+    }
     auto kern = prism::conv_unit_gates_kernel;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int threads = C >= 2048 ? 1024 : (C >= 512 ? 256 : 128);          // a few channels a thread: their loads are one chain each
