@@ -22,8 +22,14 @@
 // experts have few tiles).
 //
 // A decode step (a few rows per expert) reads every chosen expert's weights once; a prompt's tiles of one expert
-// re-read them from L2.  Every mbarrier wait is bounded, as in gemm_tcgen05.cu.
+// re-read them from L2, and that is what bounds them: a k-block of a 128 x 64 tile brings 24 KB for a million
+// multiply-adds' worth of MMA time far below its way from L2.  So the
+// gate and up product takes tiles of 128 rows where the experts have rows enough (brought in boxes of 64, only those that
+// hold rows; the MMA's N is the rows rounded up to 16): 1,999 tokens, 8 experts of 2 x 1,184 x 4,096, 2 identity
+// experts: 147 -> 109 us.  256 rows took 127 us (160 CTAs on 148 SMs), and the down product, with K of 1,184, gains nothing.  Every mbarrier wait is bounded, as in gemm_tcgen05.cu.
 #include "tcgen05.cuh"
+
+#include <type_traits>
 
 namespace prism {
 namespace tc {
@@ -46,13 +52,14 @@ template <bool CLAMP> __device__ __forceinline__ float moe_tc_glu(float g, float
 
 template <int NTOK, bool DUAL> struct MoeCfg {
     static constexpr int W_TILES = DUAL ? 2 : 1;
+    static constexpr int BOX = NTOK < 64 ? NTOK : 64;      // rows of x a copy brings
     static constexpr int STAGE_BYTES = W_TILES * MOE_TILE_M * TILE_K * 2 + NTOK * TILE_K * 2;
     // the down product of a prompt's tiles (K = an expert's inner width: few k-blocks, 64 rows to scatter): a short ring,
     // so that three CTAs share an SM and one's store hides behind the others' products; decode steps stream weights
-    // and keep the deep ring
-    static constexpr int FIT = ((DUAL || NTOK < 64) ? 200 : 72) * 1024 / STAGE_BYTES;
+    // and keep the deep ring; tiles of 128 rows (gate and up): two CTAs an SM, for the same reason
+    static constexpr int FIT = (NTOK == 128 ? 100 : (DUAL || NTOK < 64) ? 200 : 72) * 1024 / STAGE_BYTES;
     static constexpr int STAGES = FIT >= 6 ? 6 : (FIT >= 2 ? FIT : 2);
-    static constexpr int TMEM_COLS = (W_TILES * NTOK) <= 32 ? 32 : ((W_TILES * NTOK) <= 64 ? 64 : 128);
+    static constexpr int TMEM_COLS = (W_TILES * NTOK) <= 32 ? 32 : ((W_TILES * NTOK) <= 64 ? 64 : (W_TILES * NTOK) <= 128 ? 128 : W_TILES * NTOK);
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
 };
 
@@ -120,6 +127,7 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int w_row0 = e * (DUAL ? 2 : 1) * N + m_in;
     const CUtensorMap* mw = shared_tile ? &map_sw : &map_w;
     const CUtensorMap* mx = shared_tile ? &map_sx : &map_x;
+    const int boxes = (valid + C::BOX - 1) / C::BOX;       // of x's rows
     const int total_kb = (K + TILE_K - 1) / TILE_K, per_split = (total_kb + (int)gridDim.z - 1) / (int)gridDim.z;
     const int kb0 = min(total_kb, (int)blockIdx.z * per_split), nkb = min(total_kb, kb0 + per_split) - kb0;
 
@@ -141,12 +149,13 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const int s = i % STAGES;
                 if (i >= STAGES && !mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1, abortp)) break;
                 unsigned char* st = tiles + (size_t)s * C::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
+                mbar_expect_tx(&full_bar[s], W_TILES * MOE_TILE_M * TILE_K * 2 + boxes * C::BOX * TILE_K * 2);
                 const int kc = (kb0 + i) * TILE_K;
 #pragma unroll
                 for (int w = 0; w < W_TILES; ++w)
                     tma_load_2d(st + w * MOE_TILE_M * TILE_K * 2, mw, &full_bar[s], kc, w_row0 + w * N);
-                tma_load_2d(st + W_TILES * MOE_TILE_M * TILE_K * 2, mx, &full_bar[s], kc, row0);
+                for (int x = 0; x < boxes; ++x)
+                    tma_load_2d(st + (W_TILES * MOE_TILE_M + x * C::BOX) * TILE_K * 2, mx, &full_bar[s], kc, row0 + x * C::BOX);
                 issued = i + 1;
             }
             if (*abortp) {
@@ -155,8 +164,8 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) |
-                                       ((uint32_t)(MOE_TILE_M >> 4) << 24);
+            const uint32_t cols = NTOK <= 64 ? NTOK : (valid + 15) / 16 * 16;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((cols >> 3) << 17) | ((uint32_t)(MOE_TILE_M >> 4) << 24);
             bool ok = true;
             for (int i = 0; i < nkb && ok; ++i) {
                 const int s = i % STAGES;
@@ -187,7 +196,37 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         asm volatile("bar.sync 1, 128;" ::: "memory");
         const bool go = *abortp == 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (go) {
+        // rows n0 .. n0 + COLS - 1 of the tile
+        auto finish_rows = [&](const auto& acc, int n0, auto cols) {
+            if (m < N) {
+#pragma unroll
+                for (int n = 0; n < decltype(cols)::value; ++n) {
+                    if (n0 + n >= valid) continue;
+                    const int p = row0 + n0 + n;
+                    if (shared_tile && !DUAL) {
+                        reinterpret_cast<float*>(y)[(size_t)p * ldy + m] = acc[0][n];
+                    } else if (DUAL) {
+                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] =
+                            __float2bfloat16_rn(moe_tc_glu<CLAMP>(acc[0][n], acc[W_TILES - 1][n], act, limit));
+                    } else if (row_dst == nullptr) {          // an expert without a gate: its hidden layer, act(up a_p)
+                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(moe_tc_act(acc[0][n], act));
+                    } else {
+                        const float v = row_w != nullptr ? acc[0][n] * row_w[p] : acc[0][n];
+                        reinterpret_cast<float*>(y)[(size_t)row_dst[p] * ldy + m] = v;
+                    }
+                }
+            }
+        };
+        if constexpr (NTOK > 64) {                       // K is never split here
+            if (go && nkb > 0)
+                for (int n0 = 0; n0 < valid; n0 += 32) {
+                    float acc[W_TILES][32];
+#pragma unroll
+                    for (int w = 0; w < W_TILES; ++w)
+                        tmem_load<32>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + n0, acc[w]);
+                    finish_rows(acc, n0, std::integral_constant<int, 32>());
+                }
+        } else if (go) {
             float acc[W_TILES][NTOK];
 #pragma unroll
             for (int w = 0; w < W_TILES; ++w) {
@@ -232,24 +271,7 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         }
                 }
             }
-            if (finish && m < N) {
-#pragma unroll
-                for (int n = 0; n < NTOK; ++n) {
-                    if (n >= valid) continue;
-                    const int p = row0 + n;
-                    if (shared_tile && !DUAL) {
-                        reinterpret_cast<float*>(y)[(size_t)p * ldy + m] = acc[0][n];
-                    } else if (DUAL) {
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] =
-                            __float2bfloat16_rn(moe_tc_glu<CLAMP>(acc[0][n], acc[W_TILES - 1][n], act, limit));
-                    } else if (row_dst == nullptr) {          // an expert without a gate: its hidden layer, act(up a_p)
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(moe_tc_act(acc[0][n], act));
-                    } else {
-                        const float v = row_w != nullptr ? acc[0][n] * row_w[p] : acc[0][n];
-                        reinterpret_cast<float*>(y)[(size_t)row_dst[p] * ldy + m] = v;
-                    }
-                }
-            }
+            if (finish) finish_rows(acc, 0, std::integral_constant<int, NTOK>());
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -270,13 +292,13 @@ int moe_launch(const void* x, long long ldx, long long x_rows, const void* W, co
     CUtensorMap mw, mx;
     int rc = make_map(&mw, W, (long long)E * (DUAL ? 2 : 1) * N, K, K, MOE_TILE_M);
     if (rc) return rc;
-    rc = make_map(&mx, x, x_rows, K, ldx, NTOK);
+    rc = make_map(&mx, x, x_rows, K, ldx, C::BOX);
     if (rc) return rc;
     CUtensorMap msw = mw, msx = mx;
     if (sh.tiles > 0) {
         rc = make_map(&msw, sw, (long long)(DUAL ? 2 : 1) * sh.N, sh.K, sh.K, MOE_TILE_M);
         if (rc) return rc;
-        rc = make_map(&msx, sx, sh.rows, sh.K, ldsx, NTOK);
+        rc = make_map(&msx, sx, sh.rows, sh.K, ldsx, C::BOX);
         if (rc) return rc;
     }
     auto kern = moe_swap_kernel<NTOK, DUAL, CLAMP>;
@@ -360,9 +382,9 @@ PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void
     using namespace prism::tc;
     if (token_tiles <= 0 || N <= 0) return 0;
     if (E < 1 || K < 8 || K % 8 || lda % 8 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || token_tiles > 65535 ||
-        (ntok != 16 && ntok != 32 && ntok != 64))
+        (ntok != 16 && ntok != 32 && ntok != 64 && !(ntok == 128 && dual)))
         return (int)cudaErrorInvalidValue;
-    if (ksplit < 1 || ksplit > 64 || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
+    if (ksplit < 1 || ksplit > (ntok > 64 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
     if (shared_rows > 0 && (sw == nullptr || sx == nullptr || sy == nullptr || sN < 1 || sK < 8 || sK % 8 || ldsx % 8 ||
                             ((uintptr_t)sw & 15) || ((uintptr_t)sx & 15) || (!dual && row_dst == nullptr)))
         return (int)cudaErrorInvalidValue;
@@ -372,6 +394,7 @@ PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void
     if (token_tiles + sh.tiles > 65535) return (int)cudaErrorInvalidValue;
     const long long x_rows = (long long)token_tiles * ntok;
 #define ARGS a, lda, x_rows, w, offs, counts, row_dst, row_w, token_tiles, E, N, K, act, out, ldo, err, sw, sx, ldsx, sh, ksplit, ws, counters, limit, stream
+    if (ntok == 128) return act == 4 ? moe_launch<128, true, true>(ARGS) : moe_launch<128, true>(ARGS);
     if (dual && act == 4)        // the clamped form (common.cuh: clamped_glu)
         return ntok == 16 ? moe_launch<16, true, true>(ARGS) : ntok == 32 ? moe_launch<32, true, true>(ARGS) : moe_launch<64, true, true>(ARGS);
     if (dual) return ntok == 16 ? moe_launch<16, true>(ARGS) : ntok == 32 ? moe_launch<32, true>(ARGS) : moe_launch<64, true>(ARGS);

@@ -2410,6 +2410,10 @@ def moe_feed_forward(ctx, x: torch.Tensor, logits: torch.Tensor, gate_up_w: torc
     if x.dtype == torch.bfloat16 and moe_tensor_cores and L.prism_moe_tcgen05_supported(W, F) and x.stride(0) % 8 == 0:
         # tensor cores: every expert's rows start at a multiple of the token tile, one tile has one expert
         ntok = 16 if T <= 16 else (32 if T <= 32 else 64)
+        # a prompt's gate and up product reads less through tiles of 128 rows, from 256 rows an expert on (2,048 tokens, 2 of 8
+        # experts of 2 x 672 x 2,048, the whole call: 172 -> 132 us; 700 tokens: 83 and 88 us)
+        pair = 2 if gated and rows >= 256 * E else 1
+        ntok *= pair
         tiles = min(rows, (rows + E * (ntok - 1)) // ntok)          # no more tiles than this, whatever the choice
         padded = tiles * ntok
         ints = torch.empty(Z + (Z + 1) + 2 * rows + padded, dtype=torch.int32, device=dev)
@@ -2442,7 +2446,7 @@ def moe_feed_forward(ctx, x: torch.Tensor, logits: torch.Tensor, gate_up_w: torc
                                         gt, MOE_ACTS[act], _ptr(hidden), F, _ptr(err), *s1, k1, _ptr(ws), _ptr(cnt), float(limit), _stream()),
                "moe_gemm_tcgen05")
         _check(L.prism_moe_gemm_tcgen05(_ptr(hidden), F, _ptr(down_w), _ptr(offs), _ptr(counts), _ptr(row_dst),
-                                        None if scale_input else _ptr(row_w), ntok, tiles, E, W, F, 0, 0, _ptr(y), W, _ptr(err),
+                                        None if scale_input else _ptr(row_w), ntok // pair, tiles * pair, E, W, F, 0, 0, _ptr(y), W, _ptr(err),
                                         *s2, k2, _ptr(ws), _ptr(cnt), 0.0, _stream()), "moe_gemm_tcgen05")
         return y
     ints = torch.empty(Z + (Z + 1) + 4 * rows, dtype=torch.int32, device=dev)

@@ -560,6 +560,30 @@ def test_experts_on_tensor_cores_against_cuda_cores(T, W, F, E, top):
         assert float((got - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("T, W, F, E, top", [(600, 192, 136, 4, 2), (900, 128, 264, 3, 1), (1030, 72, 128, 8, 2), (256, 64, 40, 1, 1)])
+def test_experts_in_tiles_of_128_rows(T, W, F, E, top):
+    """256 rows an expert and more: stretches of several tiles, part-filled ones, an expert without a token, against the
+    CUDA-core kernels on the same choice.  Bound as above (bfloat16 hidden layers)."""
+    from prism_b200 import ops
+    g = torch.Generator().manual_seed(T + E)
+    x = torch.randn(T, W, generator=g).to(torch.bfloat16).to(DEV)
+    logits = (torch.randn(T, E, generator=g) * 2.0).to(DEV)
+    if E > 3:
+        logits[:, 1] = -30.0
+    gu = (torch.randn(E, 2 * F, W, generator=g) / W ** 0.5).to(torch.bfloat16).to(DEV)
+    dn = (torch.randn(E, W, F, generator=g) / F ** 0.5).to(torch.bfloat16).to(DEV)
+    ctx = step_ctx([T], [0])
+    for kw in (dict(), dict(softmax=True, renorm=True, scale_input=False, act="clamped", limit=0.7)):
+        ops.moe_tensor_cores = False
+        try:
+            ref = ops.moe_feed_forward(ctx, x, logits, gu, dn, top, **kw).clone()
+        finally:
+            ops.moe_tensor_cores = True
+        got = ops.moe_feed_forward(ctx, x, logits, gu, dn, top, **kw)
+        ops.check_tc_errors()
+        assert float((got - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
+
+
 # ---------------------------------------------------------------------------------------------------------
 # the model through the engine's step function
 # ---------------------------------------------------------------------------------------------------------
