@@ -220,21 +220,32 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (finish && m < N) {
                 const float b = bias != nullptr && (EPI != EPI_PARTIAL || blockIdx.y == 0) ? load_param(bias, bias_bf16, m) : 0.f;
                 const float bu = EPI == EPI_SWIGLU && bias != nullptr ? load_param(bias, bias_bf16, N + m) : 0.f;
+                // eight tokens' values side by side, then their stores: a test of every token in between would leave
+                // one chain of exponential and division per token (18,944 pairs of 3,584: 64 tokens 54.0 -> 47.2 us, 16 tokens 43.6 ->
+                // 42.0, in a decode step of 64 requests 70 -> 54; 3,584 of 18,944 as partial sums, 64 tokens: 32 -> 26)
 #pragma unroll
-                for (int n = 0; n < NTOK; ++n) {
-                    if (n >= M) continue;
-                    if (EPI == EPI_SWIGLU) {
-                        const float g = acc[0][n] + b, u = acc[W_TILES - 1][n] + bu;
-                        const float a = glu_act == 1 ? 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)))
-                                                     : g / (1.f + expf(-g));
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)n * ldy + m] =
-                            __float2bfloat16_rn(glu_act == 2 ? clamped_glu(g, u, glu_limit) : a * u);
-                    } else if (EPI == EPI_PARTIAL) {
-                        reinterpret_cast<float*>(y)[((size_t)blockIdx.y * M + n) * ldy + m] = acc[0][n] + b;
-                    } else if (EPI == EPI_F32) {
-                        reinterpret_cast<float*>(y)[(size_t)n * ldy + m] = acc[0][n] + b;
-                    } else {
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)n * ldy + m] = __float2bfloat16_rn(acc[0][n] + b);
+                for (int n0 = 0; n0 < NTOK; n0 += 8) {
+                    if (n0 >= M) break;
+                    float v[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int n = n0 + j;
+                        if (EPI == EPI_SWIGLU) {
+                            const float g = acc[0][n] + b, u = acc[W_TILES - 1][n] + bu;
+                            v[j] = glu_act == 2 ? clamped_glu(g, u, glu_limit)
+                                                : u * (glu_act == 1 ? 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)))
+                                                                    : g / (1.f + expf(-g)));
+                        } else {
+                            v[j] = acc[0][n] + b;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int n = n0 + j;
+                        if (n >= M) continue;
+                        if (EPI == EPI_PARTIAL) reinterpret_cast<float*>(y)[((size_t)blockIdx.y * M + n) * ldy + m] = v[j];
+                        else if (EPI == EPI_F32) reinterpret_cast<float*>(y)[(size_t)n * ldy + m] = v[j];
+                        else reinterpret_cast<__nv_bfloat16*>(y)[(size_t)n * ldy + m] = __float2bfloat16_rn(v[j]);
                     }
                 }
             }

@@ -192,27 +192,44 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         pdl_wait();
         const int* row_dst = pdl_fresh(row_dst_in);
         const float* row_w = pdl_fresh(row_w_in);
+        // where the tile's rows go and what they are multiplied by, a row a lane, while the products run (DUAL: not used)
+        constexpr int HOLD = DUAL ? 1 : (NTOK + 31) / 32;
+        int to[HOLD];
+        float by[HOLD];
+#pragma unroll
+        for (int k = 0; k < HOLD; ++k) {
+            const int n = lane + 32 * k, p = row0 + n;
+            to[k] = !DUAL && !shared_tile && row_dst != nullptr && n < valid ? row_dst[p] : p;
+            by[k] = !DUAL && !shared_tile && row_dst != nullptr && row_w != nullptr && n < valid ? row_w[p] : 1.f;
+        }
         if (nkb > 0) mbar_wait(acc_bar, 0, abortp);
         asm volatile("bar.sync 1, 128;" ::: "memory");
         const bool go = *abortp == 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // rows n0 .. n0 + COLS - 1 of the tile
         auto finish_rows = [&](const auto& acc, int n0, auto cols) {
-            if (m < N) {
+            // eight rows' values side by side, then their stores (as in gemm_tcgen05.cu)
 #pragma unroll
-                for (int n = 0; n < decltype(cols)::value; ++n) {
-                    if (n0 + n >= valid) continue;
-                    const int p = row0 + n0 + n;
-                    if (shared_tile && !DUAL) {
-                        reinterpret_cast<float*>(y)[(size_t)p * ldy + m] = acc[0][n];
-                    } else if (DUAL) {
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] =
-                            __float2bfloat16_rn(moe_tc_glu<CLAMP>(acc[0][n], acc[W_TILES - 1][n], act, limit));
-                    } else if (row_dst == nullptr) {          // an expert without a gate: its hidden layer, act(up a_p)
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(moe_tc_act(acc[0][n], act));
+            for (int j0 = 0; j0 < decltype(cols)::value; j0 += 8) {
+                if (n0 + j0 >= valid) break;
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float a = acc[0][j0 + j];
+                    if (DUAL) v[j] = moe_tc_glu<CLAMP>(a, acc[W_TILES - 1][j0 + j], act, limit);
+                    else if (!shared_tile && row_dst == nullptr) v[j] = moe_tc_act(a, act);
+                    else v[j] = a;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int n = n0 + j0 + j, p = row0 + n;
+                    const bool live = n < valid && m < N;
+                    if (DUAL || (!shared_tile && row_dst == nullptr)) {       // a hidden layer; without a gate act(up a_p)
+                        if (live) reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(v[j]);
                     } else {
-                        const float v = row_w != nullptr ? acc[0][n] * row_w[p] : acc[0][n];
-                        reinterpret_cast<float*>(y)[(size_t)row_dst[p] * ldy + m] = v;
+                        const int dst = __shfl_sync(0xffffffffu, to[(j0 + j) / 32 % HOLD], (j0 + j) % 32);
+                        const float wt = __shfl_sync(0xffffffffu, by[(j0 + j) / 32 % HOLD], (j0 + j) % 32);
+                        if (live) reinterpret_cast<float*>(y)[(size_t)dst * ldy + m] = v[j] * wt;
                     }
                 }
             }
