@@ -16,7 +16,7 @@
 // per SM).
 //
 //   warp 0: TMA producer      warp 1: TMEM allocation + MMA issue
-//   warps 2-5: epilogue (each reads the 32 accumulator lanes it may access)
+//   warps 2-5 (2-9 with 32 tokens and more): epilogue (each reads the 32 accumulator lanes it may access)
 //
 // Epilogues: bf16 or float32 output with optional bias; partial sums of a
 // K-split (grid.y) as float32 [split, M, N] for the next kernel to add (the
@@ -33,12 +33,16 @@ namespace prism {
 namespace tc {
 
 constexpr int TILE_M = 128;          // weight rows per CTA tile (UMMA M)
-constexpr int THREADS = 192;         // 6 warps
 
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_PARTIAL = 3 };
 
 template <int NTOK, int EPI> struct Cfg {
     static constexpr int W_TILES = EPI == EPI_SWIGLU ? 2 : 1;
+    // epilogue warps: four, or eight that share the tokens by halves where there are 32 and more, since the last tile's
+    // epilogue hides behind nothing (18,944 pairs of 3,584, 64 tokens: 47.2 -> 45.2 us; 8,192 of 2,048: 20.1 -> 17.6)
+    static constexpr int EPI_WARPS = NTOK >= 32 ? 8 : 4;
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+    static constexpr int TOK = NTOK * 4 / EPI_WARPS;       // tokens an epilogue thread has
     static constexpr int STAGE_BYTES = W_TILES * TILE_M * TILE_K * 2 + NTOK * TILE_K * 2;
     static constexpr int FIT = 208 * 1024 / STAGE_BYTES;
     static constexpr int STAGES = FIT >= 6 ? 6 : (FIT >= 2 ? FIT : 2);
@@ -47,7 +51,7 @@ template <int NTOK, int EPI> struct Cfg {
 };
 
 template <int NTOK, int EPI>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__((Cfg<NTOK, EPI>::THREADS))
 gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const void* __restrict__ bias, int bias_bf16, void* __restrict__ y, int ldy, int M, int N, int K,
                  int kblocks_per_split, int pair_offset, float* __restrict__ ws, int* __restrict__ counters, int* err,
@@ -55,6 +59,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     using C = Cfg<NTOK, EPI>;
     constexpr int W_TILES = C::W_TILES;
     constexpr int STAGES = C::STAGES;
+    constexpr int TOK = C::TOK;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * C::STAGE_BYTES);
@@ -156,25 +161,25 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             umma_commit(acc_bar);                    // the accumulator is complete (or as far as it got)
         }
     } else {
-        // ---- epilogue: warps 2..5, TMEM lanes (warp % 4) * 32 .. + 31 -----------------
-        const int q = warp & 3;
+        // ---- epilogue: warps 2 on, TMEM lanes (warp % 4) * 32 .. + 31, tokens first .. first + TOK - 1 ----
+        const int q = warp & 3, first = (warp - 2) / 4 * TOK;
         const int m = m0 + q * 32 + lane;            // this thread's output feature
         pdl_wait();                                      // outputs, bias, workspace: ordered after earlier kernels
         if (nkb > 0) mbar_wait(acc_bar, 0, abortp);      // on expiry this sets the abort flag
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps agree on the flag
+        asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");   // the epilogue warps agree on the flag
         const bool go = *abortp == 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (go) {
-            float acc[W_TILES][NTOK];
+            float acc[W_TILES][TOK];
             if (nkb > 0) {
 #pragma unroll
                 for (int w = 0; w < W_TILES; ++w)
-                    tmem_load<NTOK>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK, acc[w]);
+                    tmem_load<TOK>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + first, acc[w]);
             } else {
 #pragma unroll
                 for (int w = 0; w < W_TILES; ++w)
 #pragma unroll
-                    for (int n = 0; n < NTOK; ++n) acc[w][n] = 0.f;
+                    for (int n = 0; n < TOK; ++n) acc[w][n] = 0.f;
             }
             bool finish = true;
             if (EPI != EPI_PARTIAL && (EPI != EPI_SWIGLU || NTOK == 16) && gridDim.y > 1) {
@@ -186,16 +191,16 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
                     for (int w = 0; w < W_TILES; ++w)
 #pragma unroll
-                        for (int n = 0; n < NTOK; ++n)
-                            if (n < M) ws[(((size_t)blockIdx.y * W_TILES + w) * M + n) * N + m] = acc[w][n];
+                        for (int n = 0; n < TOK; ++n)
+                            if (first + n < M) ws[(((size_t)blockIdx.y * W_TILES + w) * M + first + n) * N + m] = acc[w][n];
                 __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");            // the four epilogue warps
+                asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");   // the epilogue warps
                 if (threadIdx.x == 64) {
                     const int old = atomicAdd(&counters[blockIdx.x], 1);
                     is_last = old == (int)gridDim.y - 1;
                     if (is_last) counters[blockIdx.x] = 0;                 // ready for the next launch
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_WARPS * 32) : "memory");
                 finish = is_last != 0;
                 if (finish && m < N) {
                     __threadfence();
@@ -203,16 +208,16 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
                     for (int w = 0; w < W_TILES; ++w)
 #pragma unroll
-                        for (int n = 0; n < NTOK; ++n) acc[w][n] = 0.f;
+                        for (int n = 0; n < TOK; ++n) acc[w][n] = 0.f;
                     for (int sp = 0; sp < (int)gridDim.y; ++sp) {
                         const float* part = ws + (size_t)sp * W_TILES * M * N + m;
 #pragma unroll
                         for (int w = 0; w < W_TILES; ++w) {
-                            float v[NTOK];
+                            float v[TOK];
 #pragma unroll
-                            for (int n = 0; n < NTOK; ++n) v[n] = n < M ? __ldcg(part + ((size_t)w * M + n) * N) : 0.f;
+                            for (int n = 0; n < TOK; ++n) v[n] = first + n < M ? __ldcg(part + ((size_t)w * M + first + n) * N) : 0.f;
 #pragma unroll
-                            for (int n = 0; n < NTOK; ++n) acc[w][n] += v[n];
+                            for (int n = 0; n < TOK; ++n) acc[w][n] += v[n];
                         }
                     }
                 }
@@ -224,8 +229,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 // one chain of exponential and division per token (18,944 pairs of 3,584: 64 tokens 54.0 -> 47.2 us, 16 tokens 43.6 ->
                 // 42.0, in a decode step of 64 requests 70 -> 54; 3,584 of 18,944 as partial sums, 64 tokens: 32 -> 26)
 #pragma unroll
-                for (int n0 = 0; n0 < NTOK; n0 += 8) {
-                    if (n0 >= M) break;
+                for (int n0 = 0; n0 < TOK; n0 += 8) {
+                    if (first + n0 >= M) break;
                     float v[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -241,7 +246,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                     }
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const int n = n0 + j;
+                        const int n = first + n0 + j;
                         if (n >= M) continue;
                         if (EPI == EPI_PARTIAL) reinterpret_cast<float*>(y)[((size_t)blockIdx.y * M + n) * ldy + m] = v[j];
                         else if (EPI == EPI_F32) reinterpret_cast<float*>(y)[(size_t)n * ldy + m] = v[j];
@@ -278,7 +283,7 @@ int launch(const void* W, int ldw, long long w_rows, const void* x, int ldx, con
     auto kern = gemm_swap_kernel<NTOK, EPI>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     dim3 grid((N + TILE_M - 1) / TILE_M, ksplit);
-    return (int)launch_kernel(kern, grid, dim3(THREADS), C::SMEM, stream, mw, mx, bias, bias_bf16, y, ldy, M, N, K, per,
+    return (int)launch_kernel(kern, grid, dim3(C::THREADS), C::SMEM, stream, mw, mx, bias, bias_bf16, y, ldy, M, N, K, per,
                               pair_offset, ws, counters, err, group_rows, group_tokens, glu_act, glu_limit);
 }
 
