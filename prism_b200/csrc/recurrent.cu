@@ -774,12 +774,13 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
                 const uint64_t u2 = pack2(uu, uu);
 #pragma unroll
                 for (int m = 0; m < Q; ++m) {
-                    if (MODE == PRISM_SCAN_DELTA) {
-                        S[p][2 * m] = mul2(S[p][2 * m], g2);
-                        S[p][2 * m + 1] = mul2(S[p][2 * m + 1], g2);
+                    if (MODE == PRISM_SCAN_DELTA) {    // the small product is the rounded one, not the decayed state
+                        S[p][2 * m] = mad2(S[p][2 * m], g2, mul2(k[m].x, u2));
+                        S[p][2 * m + 1] = mad2(S[p][2 * m + 1], g2, mul2(k[m].y, u2));
+                    } else {
+                        fma2(S[p][2 * m], k[m].x, u2);
+                        fma2(S[p][2 * m + 1], k[m].y, u2);
                     }
-                    fma2(S[p][2 * m], k[m].x, u2);
-                    fma2(S[p][2 * m + 1], k[m].y, u2);
                 }
             }
         } else if (MODE == PRISM_SCAN_GENERAL) {
