@@ -971,6 +971,34 @@ def test_scan_at_every_split(mode, H, dk, dv, lens):
         assert float((whole[s].double() - ref).abs().max()) <= bound, (i, bound)
 
 
+@pytest.mark.parametrize("T,dk", [(1, 128), (24, 128), (24, 64), (1, 20), (3, 200)])
+def test_general_scan_rounds_what_it_removes(T, dk):
+    """The state's update of the generalized delta rule, ``w S - c (e^T S) + k v``, rounds the small product ``c (e^T S)``
+    and the sum, not ``k v``.  With w and c of 2^-12 and ``|k v|`` of 0.7 to 2 the last token's sum is all that counts: half an
+    ulp of the state, at most 2^-24 |S|, beside terms of 2^-12 (4 roundings, and dk / 8 + 8 additions of e^T S)."""
+    from types import SimpleNamespace
+    ops = _ops()
+    H, dv, gen = 8, 64, torch.Generator().manual_seed(dk + T)
+    A, r = H * dk, lambda *s: torch.rand(*s, generator=gen)                                # noqa: E731
+    q, k, v = r(T, H, dk) - 0.5, 0.7 + 0.3 * r(T, H, dk), (1 + r(T, H, dv)) * (2 * (r(T, H, dv) > 0.5) - 1)
+    w, e = r(T, H, dk) * 2.0 ** -12, torch.nn.functional.normalize(r(T, H, dk) - 0.5, dim=-1)
+    c = r(T, H, dk) * 2.0 ** -12
+    x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(DEV)
+    ex = torch.cat([e.reshape(T, A), c.reshape(T, A)], 1).to(DEV)
+    state, out = torch.ones(1, H, dv, dk, device=DEV), torch.empty(T, H, dv, device=DEV)
+    ctx = SimpleNamespace(seg_start=torch.tensor([0, T], dtype=torch.int32, device=DEV), S=1, max_q_len=T,
+                          state_slots=torch.zeros(1, dtype=torch.int32, device=DEV))
+    ops.recurrent_scan(ops.SCAN_GENERAL, x[:, :A], x[:, A:2 * A], x[:, 2 * A:], state, ctx, H, 1, dk, dv, out,
+                       ww=w.reshape(T, A).to(DEV), ex=ex)
+    S = torch.ones(H, dk, dv, dtype=torch.float64)
+    for t in range(T):
+        es = (S * e[t].double()[:, :, None]).sum(1)
+        S = w[t].double()[:, :, None] * S - c[t].double()[:, :, None] * es[:, None] + k[t].double()[:, :, None] * v[t].double()[:, None]
+    err = (state[0].double().cpu() - S.transpose(1, 2)).abs()
+    small = 2.0 ** -12 * (4 + dk / 8 + 8) * dk ** 0.5 * 2
+    assert bool((err <= 2.0 ** -24 * (S.transpose(1, 2).abs() + small)).all())
+
+
 @pytest.mark.parametrize("G,H,dk,dv,K", [(2, 4, 128, 128, 4), (1, 2, 20, 65, 3), (3, 3, 8, 32, 1), (1, 1, 128, 40, 2)])
 @pytest.mark.parametrize("a_decay", [True, False])
 def test_convolution_of_many_tokens_in_runs(G, H, dk, dv, K, a_decay):
