@@ -550,10 +550,230 @@ template <int Q> __device__ __forceinline__ float quad_dot(const uint64_t (&x)[2
     return (p.x + p.y) + (r.x + r.y);
 }
 
-// LONG: groups of eight tokens, with the registers that their straight line code wants; else (a few tokens a request,
-// bound by the state's way in and out) token by token, with as many CTAs on an SM as keep that busy.
-template <int MODE, int R, int L, int CPT, bool LONG>
-__global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel(const ScanArgs a) {
+__device__ __forceinline__ void quad(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+
+// Padding entries of `rows` tokens' places in shared memory (rows beyond dk that the column's threads cover, columns beyond
+// the CTA's) are never written by the copies: zero them once.
+__device__ __forceinline__ void zero_padding(float* sm, int rows, int per_tok, int NV, int dk, int dkp, int ncols, int colsp) {
+    if (dkp == dk && colsp == ncols) return;
+    const int pad = NV * (dkp - dk) + (colsp - ncols);
+    for (int i = threadIdx.x; i < rows * pad; i += blockDim.x) {
+        const int slot = i / pad, c = i - slot * pad;
+        const int which = c / (dkp - dk > 0 ? dkp - dk : 1);
+        const int at = (dkp > dk && which < NV) ? which * dkp + dk + (c - which * (dkp - dk)) : NV * dkp + ncols + (c - NV * (dkp - dk));
+        sm[(size_t)slot * per_tok + at] = 0.f;
+    }
+}
+
+// w <- exp(-exp(w + w0)) of head h for `nb` tokens, per_tok apart; one warp
+__device__ __forceinline__ void decays_in_place(const ScanArgs& a, float* w, int per_tok, int nb, int h) {
+    for (int idx = threadIdx.x & 31; idx < nb * a.dk; idx += 32) {
+        const int tt = idx / a.dk, i = idx - tt * a.dk;
+        float& z = w[(size_t)tt * per_tok + i];
+        z = expf(-expf(z + load_param(a.w0, a.w0_bf16, (size_t)h * a.dk + i)));
+    }
+}
+
+constexpr int SCAN_STEP_BLOCKS = 3;          // blocks of tokens in shared memory: in use, landed, on its way
+
+// The scan of a step of few tokens a request: bound by the state's way in and out, so a thread has one column in as few
+// registers as it takes (70 to 90 for 128 rows and more, so that five CTAs and more share an SM) and the producer a short
+// loop a token.  48 heads of 128 x 128, delta rule, 64 single tokens: 84 us, by the kernel below 162 us.  Every product and
+// sum is written out as the kernel below has it, so that a request's values do not depend on which of the two ran.
+template <int MODE, int R, int L>
+__global__ void scan_step_kernel(const ScanArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int NV = scan_vectors(MODE), Q = R / 4, dkp = L * R, NBUF = SCAN_STEP_BLOCKS;
+    const int h = blockIdx.x, seg = blockIdx.y, col0 = blockIdx.z * a.cols;
+    const int s0 = a.seg_start[seg], qlen = a.seg_start[seg + 1] - s0;
+    const int dk = a.dk, dv = a.dv, TB = a.TB;
+    const int ncols = min(a.cols, dv - col0);
+    const int CT = blockDim.x - 32;                    // the last warp brings the vectors in
+    const bool producer = (int)threadIdx.x >= CT;
+    const int part = threadIdx.x % L;
+    const bool live = !producer && (int)threadIdx.x / L < ncols;
+    const int lc = live ? threadIdx.x / L : 0, col = col0 + lc;
+    const int kvh = h / a.rep;
+    const int per_tok = NV * dkp + a.colsp + 4;
+    const float* x = pdl_fresh(a.x);
+    const float* bg = pdl_fresh(a.bg);
+    const float* ww = pdl_fresh(a.ww);
+    const float* ex = pdl_fresh(a.ex);
+    zero_padding(sm, NBUF * TB, per_tok, NV, dk, dkp, ncols, a.colsp);
+    float* ub = sm + (size_t)NBUF * TB * per_tok;      // BONUS: u [dkp]
+    if (MODE == PRISM_SCAN_BONUS)
+        for (int i = threadIdx.x; i < dkp; i += blockDim.x) ub[i] = i < dk ? load_param(a.u, a.u_bf16, (size_t)h * dk + i) : 0.f;
+    __syncthreads();
+
+    auto stage = [&](int b0, int buf) {                // asks for block b0 of the segment's tokens
+        const int lane = threadIdx.x - CT;
+        const int nb = min(TB, qlen - b0);
+        float* dst0 = sm + (size_t)buf * TB * per_tok;
+        const int unit = a.vec ? 4 : 1;
+        const int nk = (dk + unit - 1) / unit, nc = (ncols + unit - 1) / unit;     // pieces per vector
+        const size_t head_q = (size_t)((MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_CHANNEL || MODE == PRISM_SCAN_TOKEN) ? kvh : h) * dk;
+        for (int tt = 0; tt < nb; ++tt) {
+            const size_t t = (size_t)(s0 + b0 + tt);
+            const float* xr = x + t * a.xs;
+            float* dst = dst0 + (size_t)tt * per_tok;
+            for (int c = lane; c < nk; c += 32) {
+                cp_async_f(dst + c * unit, xr + a.qo + head_q + c * unit, unit);
+                cp_async_f(dst + dkp + c * unit, xr + a.ko + head_q + c * unit, unit);
+                if (NV > 2) cp_async_f(dst + 2 * dkp + c * unit, ww + t * a.ws + (size_t)h * dk + c * unit, unit);
+                if (NV > 3) {
+                    cp_async_f(dst + 3 * dkp + c * unit, ex + t * a.es + (size_t)h * dk + c * unit, unit);
+                    cp_async_f(dst + 4 * dkp + c * unit, ex + t * a.es + (size_t)(a.H + h) * dk + c * unit, unit);
+                }
+            }
+            for (int c = lane; c < nc; c += 32)
+                cp_async_f(dst + NV * dkp + c * unit, xr + a.vo + (size_t)h * dv + col0 + c * unit, unit);
+            if ((MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_TOKEN) && lane < 2)  // beta (or dt), then g
+                cp_async_f(dst + NV * dkp + a.colsp + lane, bg + t * 2 * a.H + (size_t)lane * a.H + h, 1);
+            if (MODE == PRISM_SCAN_CHANNEL && lane == 0)                             // beta
+                cp_async_f(dst + NV * dkp + a.colsp, bg + t * a.H + h, 1);
+        }
+        cp_async_commit();
+    };
+    auto finish = [&](int b0, int buf) {               // the block has landed: the decay from its exponent
+        if (MODE == PRISM_SCAN_BONUS && !a.w_ready) {
+            __syncwarp();
+            decays_in_place(a, sm + (size_t)buf * TB * per_tok + 2 * dkp, per_tok, min(TB, qlen - b0), h);
+        }
+    };
+
+    float S[R];
+    float* st = a.state + (((size_t)a.slots[seg] * a.H + h) * dv + col) * dk;
+    if (producer) {
+        stage(0, 0);
+        if (TB < qlen) stage(TB, 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        finish(0, 0);
+    } else {
+#pragma unroll
+        for (int m = 0; m < Q; ++m) {
+            const int i = 4 * (part + L * m);
+            if (live && a.vec && i + 3 < dk) {
+                const float4 v = *reinterpret_cast<const float4*>(st + i);
+                S[4 * m] = v.x, S[4 * m + 1] = v.y, S[4 * m + 2] = v.z, S[4 * m + 3] = v.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) S[4 * m + j] = (live && i + j < dk) ? st[i + j] : 0.f;
+            }
+        }
+    }
+    __syncthreads();
+    const float keep = MODE == PRISM_SCAN_RETAIN ? load_param(a.w0, a.w0_bf16, h) : 0.f;
+    const float skip = MODE == PRISM_SCAN_TOKEN && a.w0 != nullptr ? load_param(a.w0, a.w0_bf16, h) : 0.f;
+
+    int buf = 0;
+    for (int b0 = 0; b0 < qlen; b0 += TB, buf = buf + 1 == NBUF ? 0 : buf + 1) {
+        const int nb = min(TB, qlen - b0);
+        if (producer) {
+            // the block after the next goes into the buffer freed at the last barrier; the next one is seen in
+            const int nxt = buf + 1 == NBUF ? 0 : buf + 1, nxt2 = nxt + 1 == NBUF ? 0 : nxt + 1;
+            if (b0 + 2 * TB < qlen) stage(b0 + 2 * TB, nxt2);
+            else cp_async_commit();
+            cp_async_wait<1>();
+            if (b0 + TB < qlen) finish(b0 + TB, nxt);
+            __syncthreads();
+            continue;
+        }
+        for (int tt = 0; tt < nb; ++tt) {
+            const float* row = sm + ((size_t)buf * TB + tt) * per_tok + 4 * part;      // this thread's quads of q (or r); k, .. dkp further on
+            const float* vv = row - 4 * part + NV * dkp;
+            const float v = vv[lc];
+            float o = 0.f;
+            if (MODE == PRISM_SCAN_BONUS) {
+                float b[4] = {0.f, 0.f, 0.f, 0.f}, c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int m = 0; m < Q; ++m) {
+                    float q[4], k[4], w[4], u[4];
+                    quad(row + 4 * L * m, q), quad(row + dkp + 4 * L * m, k), quad(row + 2 * dkp + 4 * L * m, w);
+                    quad(ub + 4 * (part + L * m), u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float& s = S[4 * m + j];
+                        b[j] = fmaf(__fmul_rn(q[j], u[j]), k[j], b[j]);
+                        c[j] = fmaf(s, q[j], c[j]);
+                        s = fmaf(w[j], s, __fmul_rn(k[j], v));
+                    }
+                }
+                o = fmaf((b[0] + b[1]) + (b[2] + b[3]), v, (c[0] + c[1]) + (c[2] + c[3]));
+            } else {
+                // a column's sum against the state before the update: S^T k, or e^T S
+                float u = 0.f, g = 1.f;
+                constexpr bool DELTAS = MODE == PRISM_SCAN_DELTA || MODE == PRISM_SCAN_CHANNEL;
+                if (DELTAS || MODE == PRISM_SCAN_GENERAL) {
+                    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int m = 0; m < Q; ++m) {
+                        float k[4], w[4];
+                        quad(row + (DELTAS ? 1 : 3) * dkp + 4 * L * m, k);
+                        if (MODE == PRISM_SCAN_CHANNEL) quad(row + 2 * dkp + 4 * L * m, w);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float& s = S[4 * m + j];
+                            if (MODE == PRISM_SCAN_CHANNEL) s = __fmul_rn(s, w[j]);
+                            c[j] = fmaf(s, k[j], c[j]);
+                        }
+                    }
+                    u = column_sum<L>((c[0] + c[1]) + (c[2] + c[3]));
+                }
+                if (MODE == PRISM_SCAN_DELTA) g = vv[a.colsp + 1];
+                if (DELTAS) u = vv[a.colsp] * fmaf(-g, u, v);                          // what is written along k
+                if (MODE == PRISM_SCAN_GENERAL) u = -u;
+                if (MODE == PRISM_SCAN_RETAIN) g = keep, u = v;
+                if (MODE == PRISM_SCAN_TOKEN) g = vv[a.colsp + 1], u = __fmul_rn(vv[a.colsp], v);
+                if (MODE == PRISM_SCAN_GATED) u = v;
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int m = 0; m < Q; ++m) {
+                    float q[4], k[4], w[4], e[4];
+                    quad(row + 4 * L * m, q), quad(row + dkp + 4 * L * m, k);
+                    if (MODE == PRISM_SCAN_GATED || MODE == PRISM_SCAN_GENERAL) quad(row + 2 * dkp + 4 * L * m, w);
+                    if (MODE == PRISM_SCAN_GENERAL) quad(row + 4 * dkp + 4 * L * m, e);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float& s = S[4 * m + j];
+                        if (MODE == PRISM_SCAN_CHANNEL) s = fmaf(k[j], u, s);
+                        else if (MODE == PRISM_SCAN_GENERAL) s = fmaf(k[j], v, fmaf(w[j], s, __fmul_rn(e[j], u)));
+                        else s = fmaf(MODE == PRISM_SCAN_GATED ? w[j] : g, s, __fmul_rn(k[j], u));
+                        c[j] = fmaf(s, q[j], c[j]);
+                    }
+                }
+                o = (c[0] + c[1]) + (c[2] + c[3]);
+            }
+            o = column_sum<L>(o);
+            if (MODE == PRISM_SCAN_TOKEN) o = fmaf(skip, v, o);
+            if (live && part == 0) a.out[((size_t)(s0 + b0 + tt) * a.H + h) * dv + col] = o;
+        }
+        __syncthreads();                               // the next block has landed, and this buffer is free
+    }
+    if (live) {
+#pragma unroll
+        for (int m = 0; m < Q; ++m) {
+            const int i = 4 * (part + L * m);
+            if (a.vec && i + 3 < dk) {
+                *reinterpret_cast<float4*>(st + i) = make_float4(S[4 * m], S[4 * m + 1], S[4 * m + 2], S[4 * m + 3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (i + j < dk) st[i + j] = S[4 * m + j];
+            }
+        }
+    }
+}
+
+// The scan of a step with many tokens a request.  GROUPS: eight tokens at a time (R 8 and 16), with the registers that their
+// straight line code wants; else token by token.
+template <int MODE, int R, int L, int CPT, bool GROUPS>
+__global__ void __launch_bounds__(160, GROUPS ? 1 : (R == 32 ? 3 : 5)) scan_kernel(const ScanArgs a) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -581,18 +801,7 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
     const float* ww = pdl_fresh(a.ww);
     const float* ex = pdl_fresh(a.ex);
 
-    // padding entries of the staging buffers (rows beyond dk that the column's threads cover, columns beyond the
-    // CTA's) are never written by the copies: zero them once
-    if (dkp > dk || a.colsp > ncols) {
-        const int pad = NV * (dkp - dk) + (a.colsp - ncols);
-        for (int i = threadIdx.x; i < NBUF * TB * pad; i += blockDim.x) {
-            const int slot = i / pad, c = i - slot * pad;
-            const int which = c / (dkp - dk > 0 ? dkp - dk : 1);
-            const int at = (dkp > dk && which < NV) ? which * dkp + dk + (c - which * (dkp - dk))
-                                                    : NV * dkp + ncols + (c - NV * (dkp - dk));
-            sm[(size_t)slot * per_tok + at] = 0.f;
-        }
-    }
+    zero_padding(sm, NBUF * TB, per_tok, NV, dk, dkp, ncols, a.colsp);
     __syncthreads();
 
     // the producer warp asks for block b0 of the segment's tokens into buffer `buf`: the lanes are dealt out to the
@@ -668,15 +877,9 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
     };
     // ... and, once the copies of that block have landed (the caller has waited), turns the decay's exponent into the decay
     auto finish = [&](int b0, int buf) {
-        const int nb = min(TB, qlen - b0);
-        float* dst0 = sm + (size_t)buf * TB * per_tok;
-        __syncwarp();
         if (MODE == PRISM_SCAN_BONUS && !a.w_ready) {
-            for (int idx = lane; idx < nb * dk; idx += 32) {
-                const int tt = idx / dk, i = idx - tt * dk;
-                float* w = dst0 + (size_t)tt * per_tok + 2 * dkp + i;
-                *w = expf(-expf(*w + load_param(a.w0, a.w0_bf16, (size_t)h * dk + i)));
-            }
+            __syncwarp();
+            decays_in_place(a, sm + (size_t)buf * TB * per_tok + 2 * dkp, per_tok, min(TB, qlen - b0), h);
         }
     };
 
@@ -770,7 +973,7 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
             for (int p = 0; p < CPT; ++p) ks[p] = column_sum<L>(ks[p]);
 #pragma unroll
             for (int p = 0; p < CPT; ++p) {
-                const float uu = MODE == PRISM_SCAN_DELTA ? beta * (v[p] - g * ks[p]) : beta * (v[p] - ks[p]);
+                const float uu = beta * fmaf(-g, ks[p], v[p]);
                 const uint64_t u2 = pack2(uu, uu);
 #pragma unroll
                 for (int m = 0; m < Q; ++m) {
@@ -841,7 +1044,7 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
                 if (MODE == PRISM_SCAN_GATED) w = quad(row + 2 * dkp + 4 * L * m);
 #pragma unroll
                 for (int p = 0; p < CPT; ++p) {
-                    const float t = MODE == PRISM_SCAN_TOKEN ? dt * v[p] : v[p];
+                    const float t = MODE == PRISM_SCAN_TOKEN ? __fmul_rn(dt, v[p]) : v[p];
                     const uint64_t v2 = pack2(t, t);
                     S[p][2 * m] = mad2(w.x, S[p][2 * m], mul2(k[m].x, v2));
                     S[p][2 * m + 1] = mad2(w.y, S[p][2 * m + 1], mul2(k[m].y, v2));
@@ -854,7 +1057,7 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
         float* dst = a.out + ((size_t)(s0 + tt) * a.H + h) * dv + col;
         if (MODE == PRISM_SCAN_TOKEN)
 #pragma unroll
-            for (int p = 0; p < CPT; ++p) o[p] += skip * f1[NV * dkp + lc + p];
+            for (int p = 0; p < CPT; ++p) o[p] = fmaf(skip, f1[NV * dkp + lc + p], o[p]);
         if (CPT == 4) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1 % CPT], o[2 % CPT], o[3 % CPT]);
         else if (CPT == 2) *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1 % CPT]);
         else dst[0] = o[0];
@@ -876,7 +1079,7 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
         }
         const float* blk = sm + (size_t)buf * TB * per_tok;
         int tt = 0;
-        if constexpr (LONG) {                          // L is 8
+        if constexpr (GROUPS) {                        // L is 8
             for (; tt + 8 <= nb; tt += 8) {
                 float o[8][CPT];
                 ulonglong2 q[2][Q];
@@ -938,16 +1141,13 @@ __global__ void __launch_bounds__(160, LONG ? 1 : (R == 32 ? 3 : 5)) scan_kernel
     }
 }
 
-template <int MODE, int R, int L, int CPT = 1, bool LONG = false>
-static int launch_scan(const ScanArgs& a, int S, cudaStream_t stream) {
-    const int per_tok = scan_vectors(MODE) * a.dkp + a.colsp + 4;
-    const size_t smem = (size_t)a.NBUF * a.TB * per_tok * sizeof(float);
-    static_assert(!LONG || L == 8, "");
-    auto kern = scan_kernel<MODE, R, L, CPT, LONG>;
+static int launch_scan(void (*kern)(const ScanArgs), const ScanArgs& a, int vectors, int cpt, int S, cudaStream_t stream) {
+    const int per_tok = vectors * a.dkp + a.colsp + 4;
+    const size_t smem = ((size_t)a.NBUF * a.TB * per_tok + (a.u != nullptr ? a.dkp : 0)) * sizeof(float);      // BONUS: + u
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid(a.H, S, (a.dv + a.cols - 1) / a.cols);
-    return (int)launch_kernel(kern, grid, dim3((a.cols / CPT * a.L + 31) / 32 * 32 + 32), smem, stream, a);      // + the producer warp
+    return (int)launch_kernel(kern, grid, dim3((a.cols / cpt * a.L + 31) / 32 * 32 + 32), smem, stream, a);      // + the producer warp
 }
 
 }  // namespace prism
@@ -1097,7 +1297,7 @@ PRISM_EXPORT int prism_headnorm_gate(const float* o, const float* gate, long lon
 PRISM_EXPORT int prism_recurrent_scan(int mode, const float* x, long long x_stride, long long qo, long long ko, long long vo,
                                       const float* bg,
                                       const float* ww, long long ww_stride, const void* w0, int w0_dtype, const void* u,
-                                      int u_dtype, float* state, const int* seg_start, const int* slots, int S, int max_q_len,
+                                      int u_dtype, float* state, const int* seg_start, const int* slots, int S, int T, int max_q_len,
                                       int H, int rep, int dk, int dv, float* out, int w_ready, const float* ex,
                                       long long ex_stride, cudaStream_t stream) {
     using namespace prism;
@@ -1131,8 +1331,18 @@ PRISM_EXPORT int prism_recurrent_scan(int mode, const float* x, long long x_stri
     // not (delta: 330 and 296 us).  A few tokens a request are bound by the state's way in and out: one column a thread.
     int cpt = 1, threads = 128;
     auto ctas = [&](int cols) { return (long long)H * S * ((dv + cols - 1) / cols); };
-    const bool many = quads && L == 8 && (R == 8 || R == 16) && max_q_len >= 16;
-    if (many) {
+    // Many tokens: requests of more than 16 on average, or one whose chain of tokens (some 0.2 us each are gained) is worth more
+    // than the states of all of them lose in few and heavy CTAs.  16 heads of 128 x 128, delta rule, by the two kernels: 512
+    // tokens beside 32 single ones 284 and 190 us, 40 beside 63 58 and 112 us.  States of 50 MB and more stream from HBM and want more
+    // CTAs where two vectors a token leave little else to do (64 requests of 17 tokens, 48 heads: retain 452 and 575 us, gated 660
+    // and 610).  Beyond 128 rows only five vectors a token are worth it (8 heads of 256 x 256, general: 512 tokens 363 and 291 us,
+    // 64 requests of 17 450 and 570; delta, 16 requests of 64: 224 and 294).
+    const long long states = (long long)S * H * dk * dv;
+    const bool many = quads && max_q_len >= 16 &&
+                      (R == 32 ? scan_vectors(mode) == 5 && 30000LL * max_q_len > states
+                               : T > (scan_vectors(mode) == 2 && states > 12000000 ? 32LL : 16LL) * S || 80000LL * max_q_len > states);
+    const bool groups = many && (R == 8 || R == 16);
+    if (groups) {
         int want = 4;
         while (want < 64 && ctas(want) > 148) want *= 2;
         cpt = want <= 16 ? 1 : (want == 32 ? 2 : 4);
@@ -1149,25 +1359,44 @@ PRISM_EXPORT int prism_recurrent_scan(int mode, const float* x, long long x_stri
     a.vec = quads && cols % 4 == 0;
     const int per_tok = scan_vectors(mode) * a.dkp + a.colsp + 4;
     int tb = (24 * 1024 / 4) / per_tok;
-    tb = tb < 1 ? 1 : (tb >= 16 ? 16 : (tb >= 8 ? 8 : tb));
+    tb = tb < 1 ? 1 : (tb >= 16 ? 16 : (many && tb >= 8 ? 8 : tb));
     a.TB = tb > max_q_len ? (max_q_len < 1 ? 1 : max_q_len) : tb;      // a decode step stages one token, and CTAs are small
-    // blocks on their way cover the latency of memory at some 100 ns a token; 100 KB leave room for two CTAs an SM
-    const int blocks = (max_q_len + a.TB - 1) / a.TB;
-    a.NBUF = 100 * 1024 / (a.TB * per_tok * 4);
-    a.NBUF = a.NBUF > 8 ? 8 : a.NBUF;
-    if (a.NBUF > blocks + 1) a.NBUF = blocks + 1;
-    if (a.NBUF < 3) a.NBUF = 3;
+    a.NBUF = SCAN_STEP_BLOCKS;
+    if (many) {
+        // blocks on their way cover the latency of memory at some 100 ns a token; 100 KB leave room for two CTAs an SM
+        const int blocks = (max_q_len + a.TB - 1) / a.TB;
+        // (up to 32 rows a CTA is small, and where several share an SM the others cover it)
+        a.NBUF = (R == 4 && ctas(cols) > 296 ? 36 : 100) * 1024 / (a.TB * per_tok * 4);
+        a.NBUF = a.NBUF > 8 ? 8 : a.NBUF;
+        if (a.NBUF > blocks + 1) a.NBUF = blocks + 1;
+        if (a.NBUF < 3) a.NBUF = 3;
+    }
     // rows a thread and threads a column, both known to the compiler: (4, 1..8) up to 32 rows, (8, 8), (16, 8), (32, 8..32)
+#define PRISM_SCAN_GO(K) return launch_scan(K, a, scan_vectors(mode), cpt, S, stream)
+#define PRISM_SCAN_EIGHT(M, RR)                                                                      \
+    do {                                                                                             \
+        if (!groups) PRISM_SCAN_GO((scan_step_kernel<M, RR, 8>));                                    \
+        if (cpt == 4) PRISM_SCAN_GO((scan_kernel<M, RR, 8, 4, true>));                               \
+        if (cpt == 2) PRISM_SCAN_GO((scan_kernel<M, RR, 8, 2, true>));                               \
+        PRISM_SCAN_GO((scan_kernel<M, RR, 8, 1, true>));                                             \
+    } while (0)
+#define PRISM_SCAN_ONE(M, RR, LL)                                                                    \
+    do {                                                                                             \
+        if constexpr (RR == 4 || scan_vectors(M) == 5)                                               \
+            if (many) PRISM_SCAN_GO((scan_kernel<M, RR, LL, 1, false>));                             \
+        PRISM_SCAN_GO((scan_step_kernel<M, RR, LL>));                                                \
+    } while (0)
 #define PRISM_SCAN(M)                                                                                \
     do {                                                                                             \
-        if (R == 4) return L == 1 ? launch_scan<M, 4, 1>(a, S, stream) : L == 2 ? launch_scan<M, 4, 2>(a, S, stream)    \
-                         : L == 4 ? launch_scan<M, 4, 4>(a, S, stream) : launch_scan<M, 4, 8>(a, S, stream);           \
-        if (R == 8) return cpt == 4 ? launch_scan<M, 8, 8, 4, true>(a, S, stream) : cpt == 2 ? launch_scan<M, 8, 8, 2, true>(a, S, stream) \
-                         : many ? launch_scan<M, 8, 8, 1, true>(a, S, stream) : launch_scan<M, 8, 8>(a, S, stream);                                       \
-        if (R == 16) return cpt == 4 ? launch_scan<M, 16, 8, 4, true>(a, S, stream) : cpt == 2 ? launch_scan<M, 16, 8, 2, true>(a, S, stream) \
-                         : many ? launch_scan<M, 16, 8, 1, true>(a, S, stream) : launch_scan<M, 16, 8>(a, S, stream);                                      \
-        return L == 8 ? launch_scan<M, 32, 8>(a, S, stream) : L == 16 ? launch_scan<M, 32, 16>(a, S, stream)           \
-                      : launch_scan<M, 32, 32>(a, S, stream);                                        \
+        if (R == 8) PRISM_SCAN_EIGHT(M, 8);                                                          \
+        if (R == 16) PRISM_SCAN_EIGHT(M, 16);                                                        \
+        if (R == 4 && L == 1) PRISM_SCAN_ONE(M, 4, 1);                                               \
+        if (R == 4 && L == 2) PRISM_SCAN_ONE(M, 4, 2);                                               \
+        if (R == 4 && L == 4) PRISM_SCAN_ONE(M, 4, 4);                                               \
+        if (R == 4) PRISM_SCAN_ONE(M, 4, 8);                                                         \
+        if (L == 8) PRISM_SCAN_ONE(M, 32, 8);                                                        \
+        if (L == 16) PRISM_SCAN_ONE(M, 32, 16);                                                      \
+        PRISM_SCAN_ONE(M, 32, 32);                                                                   \
     } while (0)
     if (mode == PRISM_SCAN_DELTA) PRISM_SCAN(PRISM_SCAN_DELTA);
     if (mode == PRISM_SCAN_BONUS) PRISM_SCAN(PRISM_SCAN_BONUS);
@@ -1177,5 +1406,8 @@ PRISM_EXPORT int prism_recurrent_scan(int mode, const float* x, long long x_stri
     if (mode == PRISM_SCAN_TOKEN) PRISM_SCAN(PRISM_SCAN_TOKEN);
     if (mode == PRISM_SCAN_GATED) PRISM_SCAN(PRISM_SCAN_GATED);
 #undef PRISM_SCAN
+#undef PRISM_SCAN_ONE
+#undef PRISM_SCAN_EIGHT
+#undef PRISM_SCAN_GO
     return (int)cudaErrorInvalidValue;
 }

@@ -109,7 +109,7 @@ class _Sig:
     prism_state_tail = [_p, _ll, _i, _p, _i, _p, _p, _i, _p]
     prism_shift_mix = [_p, _i, _p, _p, _i, _i, _p, _p, _p, _i, _p, _i, _ll, _i, _p]
     prism_headnorm_gate = [_p, _p, _ll, _p, _i, _i, _f, _f, _i, _i, _i, _p, _i, _ll, _i, _p]
-    prism_recurrent_scan = [_i, _p, _ll, _ll, _ll, _ll, _p, _p, _ll, _p, _i, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _i, _p, _ll, _p]
+    prism_recurrent_scan = [_i, _p, _ll, _ll, _ll, _ll, _p, _p, _ll, _p, _i, _p, _i, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _i, _p, _ll, _p]
     prism_decay_step_supported = [_i, _i]
     prism_decay_chunks_supported = [_i, _i, _i, _i]
     prism_decay_step = [_i, _p, _p, _p, _ll, _i, _i, _i, _i, _i, _i, _p, _i, _i, _f, _f, _f, _p, _p, _ll, _p, _i, _p, _i, _p, _i,
@@ -1953,7 +1953,7 @@ def recurrent_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     _check(lib().prism_recurrent_scan(
         int(mode), _ptr(q), stride, 0, k_off, v_off, _ptr(bg), _ptr(ww),
         0 if ww is None else ww.stride(0), _ptr(w0), F32 if w0 is None else _dt(w0), _ptr(u), F32 if u is None else _dt(u),
-        _ptr(state), _ptr(ctx.seg_start), _ptr(ctx.state_slots), ctx.S, int(getattr(ctx, "max_q_len", None) or T), H, rep, dk, dv,
+        _ptr(state), _ptr(ctx.seg_start), _ptr(ctx.state_slots), ctx.S, T, int(getattr(ctx, "max_q_len", None) or T), H, rep, dk, dv,
         _ptr(out), 1 if decay_ready else 0, _ptr(ex), 0 if ex is None else ex.stride(0), _stream()),
         "recurrent_scan")
 

@@ -916,7 +916,7 @@ def _scan_reference(mode, q, k, v, w, u, e, c, beta, g):
 @pytest.mark.parametrize("mode", ["delta", "bonus", "channel", "general", "retain", "token", "gated"])
 @pytest.mark.parametrize("H,dk,dv,lens", [(3, 64, 64, (37,)), (16, 128, 64, (17, 40)), (9, 100, 100, (33, 9, 16)), (16, 64, 128, (24, 3, 41))])
 def test_scan_at_every_split(mode, H, dk, dv, lens):
-    """Requests whose columns a CTA takes 8 (few heads) to 64 at a time, one to four a thread, in remainders of the
+    """Requests whose columns a CTA takes 4 (few heads) to 64 at a time, one to four a thread, in remainders of the
     blocks of eight tokens: against the recurrence in float64, and bit for bit the same when cut into single tokens
     and portions.  Bound: rounding 2^-24 of values of about 1, at most T additions deep and dk + 8 wide a token."""
     from types import SimpleNamespace
@@ -969,6 +969,57 @@ def test_scan_at_every_split(mode, H, dk, dv, lens):
         ref = _scan_reference(mode, *d)
         bound = 2.0 ** -24 * (m + dk + 8) * max(1.0, float(ref.abs().max()))
         assert float((whole[s].double() - ref).abs().max()) <= bound, (i, bound)
+
+
+@pytest.mark.parametrize("mode", ["delta", "bonus", "channel", "general", "retain", "token", "gated"])
+@pytest.mark.parametrize("H,dk,dv,long,beside", [
+    (4, 64, 64, 333, 0), (4, 128, 128, 397, 2), (16, 64, 128, 333, 3), (24, 128, 128, 333, 2), (48, 128, 128, 40, 63),
+    (2, 200, 64, 301, 1), (3, 30, 50, 301, 1), (4, 20, 32, 333, 1)])
+def test_scan_of_long_requests(mode, H, dk, dv, long, beside):
+    """A request long enough that every staging buffer is filled again several times (up to eight of 4 to 16 tokens), alone and
+    beside single tokens, which the launcher's rule gives to the kernel of many or of few tokens a request and to 8 to 64
+    columns a CTA, one to four a thread: bit for bit what the request gives in portions of 13 (below the rule), and the
+    float64 recurrence.  Bound: as above."""
+    from types import SimpleNamespace
+    ops = _ops()
+    gen = torch.Generator().manual_seed(dk + H)
+    T, A, B = long + beside, H * dk, H * dv
+    n = lambda *s: torch.randn(*s, generator=gen)                                         # noqa: E731
+    unit = lambda x: torch.nn.functional.normalize(x, dim=-1)                             # noqa: E731
+    q, k, v = unit(n(T, H, dk)), unit(n(T, H, dk)), n(T, H, dv)
+    w = 0.9 + 0.1 * torch.rand(T, H, dk, generator=gen)
+    e, u = unit(n(T, H, dk)), n(H, dk)
+    c = e * torch.rand(T, H, dk, generator=gen)
+    beta, g = torch.rand(T, H, generator=gen), 0.9 + 0.1 * torch.rand(T, H, generator=gen)
+    if mode in ("retain", "token"):
+        u[:, :] = 0.9 + 0.1 * torch.rand(H, 1, generator=gen)
+    x = torch.cat([t.reshape(T, -1) for t in (q, k, v)], 1).to(DEV)
+    kw = {"delta": dict(bg=torch.cat([beta, g], 1)), "token": dict(bg=torch.cat([beta, g], 1), w0=u[:, 0]),
+          "bonus": dict(ww=w.reshape(T, A), w0=torch.zeros(A), u=u.reshape(A), decay_ready=True),
+          "channel": dict(bg=beta, ww=w.reshape(T, A)), "gated": dict(ww=w.reshape(T, A)), "retain": dict(w0=u[:, 0]),
+          "general": dict(ww=w.reshape(T, A), ex=torch.cat([e.reshape(T, A), c.reshape(T, A)], 1))}[mode]
+    kw = {a: b if isinstance(b, bool) else b.contiguous().to(DEV) for a, b in kw.items()}
+    code = dict(delta=ops.SCAN_DELTA, bonus=ops.SCAN_BONUS, channel=ops.SCAN_CHANNEL, general=ops.SCAN_GENERAL,
+                retain=ops.SCAN_RETAIN, token=ops.SCAN_TOKEN, gated=ops.SCAN_GATED)[mode]
+
+    def go(at, lens, state):                 # consecutive rows from `at`, cut into requests
+        m = sum(lens)
+        ctx = SimpleNamespace(seg_start=torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV), S=len(lens), max_q_len=max(lens),
+                              state_slots=torch.arange(len(lens), dtype=torch.int32, device=DEV))
+        out = torch.empty(m, H, dv, device=DEV)
+        some = {a: b[at:at + m] if torch.is_tensor(b) and a in ("bg", "ww", "ex") else b for a, b in kw.items()}
+        xs = x[at:at + m]
+        ops.recurrent_scan(code, xs[:, :A], xs[:, A:2 * A], xs[:, 2 * A:], state, ctx, H, 1, dk, dv, out, **some)
+        return out
+
+    state, alone = (torch.zeros(r, H, dv, dk, device=DEV) for r in (1 + beside, 1))
+    whole = go(0, [long] + [1] * beside, state)
+    cut = torch.cat([go(at, [min(13, long - at)], alone) for at in range(0, long, 13)])
+    assert torch.equal(whole[:long], cut) and torch.equal(state[:1], alone)
+    d = [t.double().to(DEV) for t in (q[:long], k[:long], v[:long], w[:long], u, e[:long], c[:long], beta[:long], g[:long])]
+    ref = _scan_reference(mode, *d)
+    bound = 2.0 ** -24 * (long + dk + 8) * max(1.0, float(ref.abs().max()))
+    assert float((whole[:long].double() - ref).abs().max()) <= bound
 
 
 @pytest.mark.parametrize("T,dk", [(1, 128), (24, 128), (24, 64), (1, 20), (3, 200)])
