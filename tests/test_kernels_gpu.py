@@ -270,6 +270,27 @@ def test_gemm_tcgen05(M, N, K):
     assert int(err) == 0
 
 
+@pytest.mark.parametrize("M", [1, 2, 9, 31, 32, 48, 63])
+def test_gemm_tcgen05_split_many_ways(M):
+    """Sixteen shares of K added up inside the kernel, with token counts that leave either half of the epilogue's warps full,
+    part-filled or empty; one token through the paired epilogue.  Tolerances as above."""
+    ops = _ops()
+    N, K = 520, 8192
+    x, w, b, err = _rand((M, K), torch.bfloat16, 43), _rand((N, K), torch.bfloat16, 44, 0.05), _rand((N,), torch.bfloat16, 45), _err()
+    ref = x.float() @ w.float().T
+    scale = float(ref.abs().max())
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=DEV)
+    ops.gemm_tc(x, w, b, out[:M], ops.EPI_F32, ksplit=16, err=err)
+    assert torch.allclose(out[:M], ref + b.float(), atol=2e-3 * scale, rtol=2e-3) and bool((out[M] == 7.0).all())
+    for ks in (1, 3) if M <= 16 else (1,):
+        act = torch.full((M + 1, N // 2), 7.0, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_tc(x, w, None, act[:M], ops.EPI_SWIGLU, ksplit=ks, err=err)
+        g, u = ref[:, :N // 2], ref[:, N // 2:]
+        r = g * torch.sigmoid(g) * u
+        assert torch.allclose(act[:M].float(), r, atol=1e-2 * float(r.abs().max()) + 1e-3, rtol=2e-2) and bool((act[M] == 7.0).all())
+    assert int(err) == 0
+
+
 def test_split_k_workspace_outgrown_after_a_graph_was_captured():
     """A graph captured with the K-split product's workspace keeps replaying correctly after a later eager
     call has outgrown that workspace: the old one stays allocated, so nobody else's data can land where the
