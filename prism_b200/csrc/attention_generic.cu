@@ -217,7 +217,7 @@ attn_generic_kernel(const T* q, int q_stride, int q_head_stride, T* out,
             sum += part[dv + 1] * f;
         }
         if (sink != nullptr) sum += expf(load_param(sink, sink_bf16, h0 + p) - top);
-        out[(size_t)t * out_stride + (size_t)(h0 + p) * dv + d] = from_float<T>(sum > 0.f ? o / sum : 0.f);
+        out[(size_t)t * out_stride + (size_t)(h0 + p) * dv + d] = from_float<T>(sum > 0.f ? o / sum : o * 0.f);      // no key: zero; not a number stays that
     }
 }
 

@@ -524,6 +524,21 @@ def test_attention_generic_in_one_order(nh, nkv, hd, window, segs, dtype):
         assert torch.equal(one[0], out[t]), t
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(6, 2, 64), (3, 3, 40)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_hides_no_nan(nh, nkv, hd, dtype):
+    """A score of infinity makes its head's output not a number, as in the plain evaluation, and leaves the others alone."""
+    ops = _ops()
+    c = PagedCase([(0, 3), (200, 2)], nh, nkv, hd, 16, dtype, seed=22)
+    c.q[3, 2, 5], c.q[4, 0, :] = float("inf"), float("nan")           # (3, 2): 201 keys, some of an infinite score
+    out, err, scale = torch.empty(c.T, nh * hd, dtype=dtype, device=DEV), _err(), hd ** -0.5
+    ops.attention_generic(c.q, out, c.k, c.v, c.bt, c.positions, c.tok_seg, c.num_pages, None, scale, err)
+    got = out.float().view(c.T, nh, hd).isnan()
+    assert bool(got[3, 2].all()) and int(err) == 0
+    got[3, 2] = got[4, 0] = False              # (every score of (4, 0) is no number: no key is seen)
+    assert not bool(got.any())
+
+
 def test_attention_generic_rejects_big_head():
     ops = _ops()
     c = PagedCase([(0, 2)], 1, 1, 272, 16, torch.float32, seed=1)
