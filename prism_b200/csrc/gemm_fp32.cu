@@ -367,10 +367,18 @@ template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC> int many(const C
 }
 
 template <bool VEC> int pick(const Call& c) {
+    auto tiles = [&](int bm, int bn) { return (long long)((c.M + bm - 1) / bm) * ((c.N + bn - 1) / bn); };
+    // A short K (few of the eight classes have a slice) leaves the few rows' lanes and the cluster's CTAs idle: small tiles,
+    // while they are no more than ten an SM (252 rows, N 2,048, K 32: 5.8 us, cluster 16.1; 512 rows, N 8,192, K 16: 14.7 us,
+    // 128 x 64 13.1).  Few rows take longer the more rows and columns they have, the tiles the longer K is (12 rows, N 4,096, K 64:
+    // 4.2 us by tiles, 13.6 by rows; 4 rows, N 512, K 128: 6.2 and 2.4).
+    int rows = 1;
+    while (rows < c.M && rows < 32) rows *= 2;
+    if (c.K <= (rows == 32 ? 3 * SLICE : (c.N < 1500 ? 3 : c.N < 4736 ? 10 : 12) * rows))
+        return tiles(32, 32) <= 1500 ? many<32, 32, 4, 4, false, VEC>(c) : many<128, 64, 8, 4, false, VEC>(c);
     if (c.M <= 16) return few_m<VEC>(c);
-    // tiles of 64 x 64 that do not fill the 148 SMs twice have their K shared by a cluster
-    const long tiles = (long)((c.M + 63) / 64) * ((c.N + 63) / 64);
-    if (tiles < 296) return many<64, 64, 4, 4, true, VEC>(c);
+    // tiles of 64 x 64 that do not fill the 148 SMs twice have their K shared by a cluster, as far as its CTAs have slices
+    if (tiles(64, 64) * PERIOD < 296LL * (c.K < PERIOD ? c.K : PERIOD)) return many<64, 64, 4, 4, true, VEC>(c);
     if (c.M <= 64) return many<64, 64, 4, 4, false, VEC>(c);
     return many<128, 64, 8, 4, false, VEC>(c);
 }

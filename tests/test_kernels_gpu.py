@@ -169,11 +169,12 @@ def test_sgemm(M, N, K):
     assert torch.equal(out1[0], out[M // 2])
 
 
-@pytest.mark.parametrize("N,K", [(7, 5), (896, 864), (130, 257), (4736, 300), (9000, 64)])
+@pytest.mark.parametrize("N,K", [(7, 5), (896, 864), (130, 257), (4736, 300), (9000, 64), (19000, 864), (8200, 128), (8200, 129),
+                                 (4100, 192), (60, 193), (33, 100)])
 @pytest.mark.parametrize("pad", [0, 1])
 def test_sgemm_same_at_every_row_count(N, K, pad):
-    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone; 16-byte and single
-    copies) adds a row's products in the same order.  Bound: K products of about 0.05, the chains at most K / 8 long."""
+    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone of three sizes with one or several
+    slices a class, a short K; 16-byte and single copies) adds a row's products in the same order.  Bound: K products of about 0.05, the chains at most K / 8 long."""
     ops = _ops()
     x = _rand((300, K + pad), torch.float32, 6)[:, :K]
     w = _rand((N, K + pad), torch.float32, 7, 0.05)[:, pad:]
