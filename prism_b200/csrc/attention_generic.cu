@@ -16,13 +16,14 @@
 // A CTA takes a token and HPW query heads of one kv head; block b of the position's keys belongs to warp b % W.
 // A lane scores one key of the block (for every head of the CTA, from one read of the key), the block's
 // probabilities are exchanged by shuffles, and a lane accumulates the output entries lane, lane + 32, ...; the W
-// warps' sums meet in shared memory in their order.  W is a constant of the value size, so the order of additions
-// stays a matter of the position alone.
+// warps' sums meet in shared memory in their order.  W is a constant of the layer (its value and key sizes and its heads per kv
+// head), never of the batch, so within a layer the order of additions stays a matter of the position alone; HPW changes no sum.
 //
 // Bound by latency (a step of few tokens: one chain of page lookup, key rows, softmax, value rows per block) or by the
 // reads of keys and values through the caches (prompts).  Hence blocks side by side, eight rows of loads in flight
 // and one read of keys and values for several heads.  14 heads over 2 of 64, float32, against one warp per head and
-// token: 3 tokens behind 100 keys 41 -> 12.5 us, 16 behind 400 142 -> 21 us, a prompt of 512 306 -> 116 us.
+// token: 3 tokens behind 100 keys 38 -> 7.2 us, 16 behind 400 139 -> 16 us, a prompt of 512 304 -> 93 us; 32 heads of 128 of their
+// own, bf16, the same prompt 682 -> 466 us.
 #include "common.cuh"
 
 namespace prism {
@@ -181,8 +182,9 @@ attn_generic_kernel(const T* q, int q_stride, int q_head_stride, T* out,
                 const T* vr = vc + (size_t)(rj < 0 ? 0 : rj) * v_row_stride + (size_t)kvh * v_head_stride;
 #pragma unroll
                 for (int i = 0; i < MAXD; ++i) {
-                    const int d = lane + 32 * i;
-                    v[e][i] = rj >= 0 && d < dv ? to_float(vr[d]) : 0.f;
+                    // always a load, of an entry that exists: a test ahead of it puts the loads one behind the other
+                    const float x = to_float(vr[min(lane + 32 * i, dv - 1)]);
+                    v[e][i] = rj >= 0 ? x : 0.f;
                 }
             }
 #pragma unroll
@@ -260,11 +262,11 @@ PRISM_EXPORT int prism_attention_masked_generic(const void* q, int q_stride, int
     if (mask_keep < 0 || (mask_keep > 0 && mask_kind != PRISM_MASK_WINDOW)) return (int)cudaErrorInvalidValue;
     if (dv > 1024 || dv <= 0 || dk <= 0 || dk > 8192 || nkv <= 0 || nh % nkv != 0) return (int)cudaErrorInvalidValue;
     const int sb = sink_dtype == PRISM_DTYPE_BF16;
-    // Four heads of a kv head a CTA wherever it has several (14 over 2 heads of 64, float32: 3 tokens behind 100 keys 12.5
-    // us, a CTA a head 13.9; a prompt of 512 117 and 234 us), with eight warps, since their blocks are the decode steps'
-    // chain (16 tokens behind 400 keys: 8 warps 22 us, 4 warps 38).  A kv head for every head: four warps (8 heads of
-    // 128, bf16, prompt of 512: 293 us, 8 warps 406; 2 tokens behind 300 keys: 59 and 36).
-    const bool wide = nh / nkv >= 2 && dk <= 512;
+    // Several heads of a kv head: eight warps, since their blocks are the decode steps' chain (14 over 2 heads of 64, float32, 16 tokens
+    // behind 400 keys: 16 us, four warps 27), and four heads a CTA (a prompt of 512: 94 us, a CTA a head 196), but one where all of them
+    // fit the 148 SMs at once and a CTA's four would follow one another (3 tokens behind 100 keys: 7.2 us, four heads 8.7; 16 behind 400
+    // have 224: 20 and 16).  A kv head for every head: four warps (8 heads of 128, bf16, prompt of 512: 139 us, 8 warps 147).
+    const bool several = nh / nkv >= 2 && dk <= 512, wide = several && (long long)T * nh > 148;
 #define PRISM_GENERIC(TT, MD, HP, WW)                                                                               \
     return prism::launch_generic<TT, MD, HP, WW>(q, q_stride, q_head_stride, out, out_stride, kc, k_row_stride,     \
                                                  k_head_stride, vc, v_row_stride, v_head_stride, block_table,       \
@@ -274,8 +276,10 @@ PRISM_EXPORT int prism_attention_masked_generic(const void* q, int q_stride, int
 #define PRISM_GENERIC_BY_SIZE(TT)                                                                                   \
     do {                                                                                                            \
         if (dv <= 64 && wide) PRISM_GENERIC(TT, 2, 4, 8);                                                           \
+        if (dv <= 64 && several) PRISM_GENERIC(TT, 2, 1, 8);                                                        \
         if (dv <= 64) PRISM_GENERIC(TT, 2, 1, 4);                                                                   \
         if (dv <= 128 && wide) PRISM_GENERIC(TT, 4, 4, 8);                                                          \
+        if (dv <= 128 && several) PRISM_GENERIC(TT, 4, 1, 8);                                                       \
         if (dv <= 128) PRISM_GENERIC(TT, 4, 1, 4);                                                                  \
         if (dv <= 256) PRISM_GENERIC(TT, 8, 1, 4);                                                                  \
         if (dv <= 512) PRISM_GENERIC(TT, 16, 1, 4);                                                                 \

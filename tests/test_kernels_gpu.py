@@ -510,7 +510,7 @@ def test_attention_generic(case, dtype):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_generic_in_one_order(nh, nkv, hd, window, segs, dtype):
     """Several heads of a kv head a CTA, or one, with remainders of heads, blocks, rows and warps: against the reference,
-    and bit for bit what a token gives alone."""
+    and bit for bit what a token gives alone (then with one head a CTA in every case)."""
     ops = _ops()
     c = PagedCase(segs, nh, nkv, hd, 16, dtype, seed=21)
     out, err, scale = torch.empty(c.T, nh * hd, dtype=dtype, device=DEV), _err(), hd ** -0.5
