@@ -114,8 +114,8 @@ __global__ void conv_unit_gates_kernel(const float* __restrict__ proj_in, long l
 // The same for a step of many tokens: a warp takes one head's channels (q, k or v; d = lane + 32 m) of RUN tokens one
 // after another with the inputs of the last K - 1 tokens and the taps in registers, so that every input is read once
 // instead of K times and nothing passes through shared memory; sums in the order of the kernel above.  One more "head"
-// forms the gates.  Bound by the bytes of proj and qkv: 2,048 tokens of 6,144 channels 78 us by the kernel above,
-// 13 us here.
+// forms the gates.  Bound by the bytes of proj and qkv (2,048 tokens of 6,144 channels, 101 MB, inputs from memory: 145 us by the
+// kernel above, 38 us here; what the projection just wrote is in L2 in part).
 constexpr int CONV_RUN = 16, CONV_TAPS = 4;
 template <int M>
 __global__ void __launch_bounds__(128) conv_unit_gates_run_kernel(const float* __restrict__ proj_in, long long ps, int ob, int oa,
@@ -1162,16 +1162,20 @@ PRISM_EXPORT int prism_conv_unit_gates(const float* proj, long long ps, int ob, 
     const int C = 2 * G * dk + H * dv;
     const size_t smem = (size_t)C * sizeof(float);
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-    // runs of tokens where there are enough of them to fill the GPU with a warp a head and run
-    const int widest = dk > dv ? dk : dv;
-    if (!move_tail && K <= prism::CONV_TAPS && widest <= 128 && T >= 256) {
+    // Runs of tokens: a warp's sixteen tokens one after another take 8 to 12 us whatever else there is, so only where the other
+    // kernel, bound by its T C channels, takes longer, and where the warps' lanes are not mostly idle (a head has 1, 2 or 4 entries a
+    // lane).  Six heads of 128: 512 tokens 8.3 us and 11.9 in runs, 1,024 11.7 and 12.7, 2,048 19.1 and 16.8; 48 of 128: 256 tokens
+    // 19.2 and 15.0; 16 of 64: 512 tokens 8.8 and 9.0, 1,024 11.8 and 10.6.
+    const int widest = dk > dv ? dk : dv, per_lane = widest <= 32 ? 1 : widest <= 64 ? 2 : 4;
+    if (!move_tail && K <= prism::CONV_TAPS && widest <= 128 && (long long)T * C >= (widest <= 64 ? 600000 : 1200000) &&
+        (2 * G + H) * 32 * per_lane <= 2 * C) {
         const dim3 grid((T + prism::CONV_RUN - 1) / prism::CONV_RUN, (2 * G + H + 1 + 3) / 4);
         auto run = [&](auto kernel) {
             return (int)prism::launch_kernel(kernel, grid, dim3(128), 0, stream, proj, ps, ob, oa, taps, taps_dtype == PRISM_DTYPE_BF16, K,
                                              tail, a_log, a_log_dtype == PRISM_DTYPE_BF16, dt_bias, dt_dtype == PRISM_DTYPE_BF16, tok_seg,
                                              seg_start, slots, T, G, H, dk, dv, unit_eps, qkv, bg);
         };
-        return widest <= 32 ? run(prism::conv_unit_gates_run_kernel<1>) : widest <= 64 ? run(prism::conv_unit_gates_run_kernel<2>)
+        return per_lane == 1 ? run(prism::conv_unit_gates_run_kernel<1>) : per_lane == 2 ? run(prism::conv_unit_gates_run_kernel<2>)
                             : run(prism::conv_unit_gates_run_kernel<4>);
     }
     auto kern = prism::conv_unit_gates_kernel;

@@ -1090,8 +1090,8 @@ def test_general_scan_rounds_what_it_removes(T, dk):
 @pytest.mark.parametrize("G,H,dk,dv,K", [(2, 4, 128, 128, 4), (1, 2, 20, 65, 3), (3, 3, 8, 32, 1), (1, 1, 128, 40, 2)])
 @pytest.mark.parametrize("a_decay", [True, False])
 def test_convolution_of_many_tokens_in_runs(G, H, dk, dv, K, a_decay):
-    """Steps of 256 tokens and more take runs of tokens per warp: bit for bit what the kernel for shorter steps gives for
-    the same requests, which begin inside runs, reach into their tails and are shorter than the convolution."""
+    """A step of several requests, which begin inside stretches of sixteen tokens, reach into their tails and are shorter than
+    the convolution: bit for bit what the same requests give alone.  (Steps wide enough for runs of tokens per warp: below.)"""
     from types import SimpleNamespace
     ops = _ops()
     C, lens = 2 * G * dk + H * dv, [2, 150, 1, 97, 31]
@@ -1112,5 +1112,34 @@ def test_convolution_of_many_tokens_in_runs(G, H, dk, dv, K, a_decay):
 
     qkv, bg = go(0, len(lens))
     assert T >= 256
+    parts = [go(i, 1) for i in range(len(lens))]
+    assert torch.equal(qkv, torch.cat([p[0] for p in parts])) and torch.equal(bg, torch.cat([p[1] for p in parts]))
+
+
+@pytest.mark.parametrize("G,H,dk,dv,K,lens", [
+    (16, 16, 128, 128, 4, [2, 90, 1, 97, 31]), (3, 5, 20, 30, 3, [1, 700, 2, 900, 650]), (2, 4, 64, 33, 1, [17, 900, 800]),
+    (1, 1, 128, 40, 2, [2000, 1, 2100]), (1, 2, 20, 65, 3, [1500, 2]), (2, 2, 8, 8, 4, [900, 300])])
+@pytest.mark.parametrize("a_decay", [True, False])
+def test_convolution_by_runs_and_by_tokens(G, H, dk, dv, K, lens, a_decay):
+    """Steps whose tokens times channels (and lanes) give them to a warp a head and run of sixteen tokens, and some that are
+    left to the kernel for shorter steps: bit for bit what the requests give alone, most of them by the latter."""
+    from types import SimpleNamespace
+    ops = _ops()
+    C, T, gen = 2 * G * dk + H * dv, sum(lens), torch.Generator().manual_seed(K)
+    proj = torch.randn(T, C + 2 * H + 3, generator=gen).to(DEV)
+    taps, tail = torch.randn(C, K, generator=gen).to(DEV), torch.randn(len(lens) + 1, K - 1, C, generator=gen).to(DEV)
+    a_log, dt = (torch.randn(H, generator=gen).to(DEV) if a_decay else None for _ in range(2))
+
+    def go(first, n):
+        start = torch.tensor([0] + lens[first:first + n]).cumsum(0)
+        ctx = SimpleNamespace(S=n, max_q_len=max(lens[first:first + n]), seg_start=start.to(torch.int32).to(DEV),
+                              tok_seg=torch.repeat_interleave(torch.arange(n), torch.tensor(lens[first:first + n])).to(torch.int32).to(DEV),
+                              state_slots=torch.arange(first + 1, first + n + 1, dtype=torch.int32, device=DEV))
+        at, m = sum(lens[:first]), int(start[-1])
+        qkv, bg = torch.empty(m, C, device=DEV), torch.empty(m, (2 if a_decay else 1) * H, device=DEV)
+        ops.conv_unit_gates(proj[at:at + m], C, C + H if a_decay else 0, taps, tail, a_log, dt, ctx, G, H, dk, dv, 1e-6, qkv, bg)
+        return qkv, bg
+
+    qkv, bg = go(0, len(lens))
     parts = [go(i, 1) for i in range(len(lens))]
     assert torch.equal(qkv, torch.cat([p[0] for p in parts])) and torch.equal(bg, torch.cat([p[1] for p in parts]))
