@@ -34,15 +34,15 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float* src, int bytes)
 
 // ---- few rows -----------------------------------------------------------------------------------------
 // A CTA owns BN weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared
-// memory stages (cp.async; the weights of the first stages are asked for before the dependency wait where the
-// caller says that no earlier kernel of the stream writes them, w_static).  Thread =
+// memory stages (cp.async; the weights of the first stages are brought into L2 before the dependency wait: read they are
+// after it, so that they may also be what an earlier kernel of the stream writes).  Thread =
 // (class, column group): the eight classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie
 // at (class, piece ^ class), so that the eight lanes read eight different bank groups.
 // BN 8 where N is small (N 896: 112 CTAs), else 32 with two columns a thread, which halves the reads of A.
 template <int MT, int BN, int CPT, int STAGES, bool VEC>
 __global__ void __launch_bounds__(BN / CPT * CLASSES)
 few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
-                int bias_bf16, float* C, int ldc, int M, int N, int K, int w_static) {
+                int bias_bf16, float* C, int ldc, int M, int N, int K) {
     constexpr int THREADS = BN / CPT * CLASSES;
     constexpr int STAGE = (BN + MT) * PERIOD;
     extern __shared__ __align__(16) float smem[];
@@ -69,16 +69,19 @@ few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __
     };
 
     pdl_trigger();
-    if (!w_static) pdl_wait();
-    W = pdl_fresh(W);
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s)
-        if (s < periods) load(W, ldw, BN, N, n0, s, smem + s * STAGE);
-    if (w_static) pdl_wait();
-    A = pdl_fresh(A);
+    // lines of 128 bytes: eight of a row a period
+    for (int idx = tid; idx < BN * 8 * (STAGES - 1); idx += THREADS) {
+        const int r = idx / (8 * (STAGES - 1)), k = idx % (8 * (STAGES - 1)) * 32;
+        if (n0 + r < N && k < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)(n0 + r) * ldw + k));
+    }
+    pdl_wait();
+    W = pdl_fresh(W), A = pdl_fresh(A);
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < periods) load(A, lda, MT, M, 0, s, smem + s * STAGE + BN * PERIOD);
+        if (s < periods) {
+            load(W, ldw, BN, N, n0, s, smem + s * STAGE);
+            load(A, lda, MT, M, 0, s, smem + s * STAGE + BN * PERIOD);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
@@ -322,7 +325,7 @@ struct Call {
     const void* bias;
     int bb;
     float* C;
-    int ldc, M, N, K, w_static;
+    int ldc, M, N, K;
     cudaStream_t stream;
 };
 
@@ -334,7 +337,7 @@ template <int MT, int BN, int CPT, int STAGES, bool VEC> int few(const Call& c) 
         if (e != cudaSuccess) return (int)e;
     }
     return (int)launch_kernel(kern, dim3((c.N + BN - 1) / BN), dim3(BN / CPT * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
-                              c.bb, c.C, c.ldc, c.M, c.N, c.K, c.w_static);
+                              c.bb, c.C, c.ldc, c.M, c.N, c.K);
 }
 
 // BN 8 keeps every SM busy down to N of about a thousand; from 148 x 32 columns on wider CTAs fill the GPU too
@@ -387,10 +390,10 @@ template <bool VEC> int pick(const Call& c) {
 }  // namespace prism
 
 PRISM_EXPORT int prism_sgemm_nt(const float* A, int lda, const float* W, int ldw, const void* bias,
-                                int bias_dtype, float* C, int ldc, int M, int N, int K, int w_static,
+                                int bias_dtype, float* C, int ldc, int M, int N, int K,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    const prism::f32gemm::Call c{A, lda, W, ldw, bias, bias_dtype == PRISM_DTYPE_BF16, C, ldc, M, N, K, w_static, stream};
+    const prism::f32gemm::Call c{A, lda, W, ldw, bias, bias_dtype == PRISM_DTYPE_BF16, C, ldc, M, N, K, stream};
     // 16-byte copies where every row starts on a 16-byte boundary
     const bool vec = ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && (M == 1 || lda % 4 == 0) && (N == 1 || ldw % 4 == 0);
     return vec ? prism::f32gemm::pick<true>(c) : prism::f32gemm::pick<false>(c);

@@ -157,7 +157,7 @@ class _Sig:
                                   _f, _p, _i, _p, _p, _i, _p]
     prism_attention_merge_bf16 = [_p, _p, _i, _p, _i, _i, _i, _i, _p]
     prism_swiglu = [_p, _p, _i, _i, _i, _p]
-    prism_sgemm_nt = [_p, _i, _p, _i, _p, _i, _p, _i, _i, _i, _i, _i, _p]
+    prism_sgemm_nt = [_p, _i, _p, _i, _p, _i, _p, _i, _i, _i, _i, _p]
     prism_sample = [_p, _i, _i, _i, _p, _p, _p, _p]
     prism_argmax_split = [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p]
     prism_set_pdl = [_i]
@@ -252,9 +252,8 @@ def add_normed_rmsnorm(residual: torch.Tensor, delta: torch.Tensor, delta_weight
            "add_normed_rmsnorm")
 
 
-def sgemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, w_static: bool = False):
-    """True float32 ``out = x @ w.T + bias`` on CUDA cores.  ``w_static``: ``w`` is a stored weight that no kernel of
-    the step writes, so it may be read before the kernels ahead in the stream have finished."""
+def sgemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor):
+    """True float32 ``out = x @ w.T + bias`` on CUDA cores."""
     _cuda(x, w, bias, out)
     assert x.dtype == torch.float32 and w.dtype == torch.float32 and out.dtype == torch.float32
     assert all(t.stride(-1) == 1 or t.shape[-1] == 1 for t in (x, w, out))
@@ -263,7 +262,7 @@ def sgemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: t
     assert w.shape[1] == K and out.shape == (M, N)
     _check(lib().prism_sgemm_nt(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias),
                                 F32 if bias is None else _dt(bias), _ptr(out), out.stride(0), M, N, K,
-                                int(w_static), _stream()), "sgemm")
+                                _stream()), "sgemm")
 
 
 USE_GEMV = os.environ.get("PRISM_GEMV", "1") != "0"
@@ -462,7 +461,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         w32 = w if w.dtype == torch.float32 else w.float()
         o32 = out if (out is not None and out.dtype == torch.float32) else \
             torch.empty((M, N), dtype=torch.float32, device=x.device)
-        sgemm(x32, w32, bias, o32, w_static=w32 is w)
+        sgemm(x32, w32, bias, o32)
         if want == torch.float32:
             return o32
         if out is not None:
@@ -1694,7 +1693,7 @@ def matmul_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
     assert w.shape[0] == H and w.shape[2] == K and out.shape == (T, H, w.shape[1])
     if x.dtype == torch.float32:
         for h in range(H):
-            sgemm(x[:, h], w[h], None, out[:, h], w_static=True)
+            sgemm(x[:, h], w[h], None, out[:, h])
         return
     torch.bmm(x.transpose(0, 1), w.transpose(1, 2), out=out.transpose(0, 1))
 

@@ -189,6 +189,30 @@ def test_sgemm_same_at_every_row_count(N, K, pad):
     assert (rows[:, :N].double() - ref).abs().max() < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
 
 
+@pytest.mark.parametrize("M", [1, 3, 16, 40])
+def test_linear_reads_a_weight_that_was_just_written(M):
+    """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
+    may be read before that kernel has ended.  Bound: two products of K terms, chains of K / 8."""
+    ops = _ops()
+    N, K = 3000, 512
+    x, b = _rand((M, K), torch.float32, 46), _rand((K, K), torch.float32, 47, 0.05)
+    w = torch.zeros(N, K, dtype=torch.float32, device=DEV)
+    outs = []
+    for i in range(12):
+        a = _rand((N, K), torch.float32, 48 + i)
+        y, z = (torch.empty(M, N, dtype=torch.float32, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        ops.sgemm(a, b, None, w)                       # 188 tiles of 128 x 64 that release what follows at once
+        ops.linear(x, w, None, out=y)
+        ops.sgemm(a, b[:, :], None, w)
+        ops.matmul_heads(x[:, None], w[None], z[:, None])
+        outs.append((a, y, z))
+    for a, y, z in outs:
+        ref = x.double() @ (a.double() @ b.double().T).T
+        bound = 2.0 ** -24 * 2 * (K / 8 + 16) * float(ref.abs().max())
+        assert float((y.double() - ref).abs().max()) <= bound and torch.equal(y, z)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 152, 96), (8, 4608, 3584), (300, 1000, 512)])
 def test_linear_bf16(M, N, K):
     ops = _ops()
