@@ -2321,6 +2321,21 @@ def _moe_ksplit(N: int, K: int, live: int) -> int:
     return max(1, min(num_sms() // (live * -(-N // 128)), (K + 63) // 64 // 8))
 
 
+def _expert_tiles(T: int, top: int, E: int, Z: int, F: int, gated: bool, sms: int) -> tuple:
+    """``(rows a tile of the gate and up product, tiles of the down product each of them is cut into, tiles)`` of a step on
+    tensor cores: ``tiles`` is no fewer than there can be, whatever the choice.  A prompt's gate and up product reads less from
+    L2 through tiles of 128 rows, two CTAs an SM, as soon as tiles of 64, which have an SM each, would not all run at once (an
+    even choice leaves an expert's last tile half full).  The whole call, tiles of 64 and of 128: 8 experts of 2 x 672 x 2,048,
+    128 rows each (120 CTAs) 63 and 75 us, 176 (156) 86 and 82, 512 155 and 135; 2 x 256 x 1,024, 512 rows (136) 61 and 68,
+    700 (183) 80 and 73; 64 experts of 2 x 1,024 x 2,048, 300 rows 763 and 611."""
+    rows = T * top
+    ntok = 16 if T <= 16 else (32 if T <= 32 else 64)
+    most = lambda n: min(rows, (rows + E * (n - 1)) // n)                              # noqa: E731
+    if gated and ntok == 64 and -(-F // 128) * (rows * E // Z / 64 + E / 2) > sms and 2 * most(128) <= 65535:
+        return 128, 2, most(128)
+    return ntok, 1, most(ntok)
+
+
 class MoeChoice:
     """How a router's scores become a choice beyond "the largest": ``correction [E]`` is added to every score for
     the choice only (the weights use the scores without it); the experts form ``groups`` equal groups of
@@ -2408,12 +2423,7 @@ def moe_feed_forward(ctx, x: torch.Tensor, logits: torch.Tensor, gate_up_w: torc
             return y
     if x.dtype == torch.bfloat16 and moe_tensor_cores and L.prism_moe_tcgen05_supported(W, F) and x.stride(0) % 8 == 0:
         # tensor cores: every expert's rows start at a multiple of the token tile, one tile has one expert
-        ntok = 16 if T <= 16 else (32 if T <= 32 else 64)
-        # a prompt's gate and up product reads less through tiles of 128 rows, from 256 rows an expert on (2,048 tokens, 2 of 8
-        # experts of 2 x 672 x 2,048, the whole call: 172 -> 132 us; 700 tokens: 83 and 88 us)
-        pair = 2 if gated and rows >= 256 * E else 1
-        ntok *= pair
-        tiles = min(rows, (rows + E * (ntok - 1)) // ntok)          # no more tiles than this, whatever the choice
+        ntok, pair, tiles = _expert_tiles(T, top, E, Z, F, gated, num_sms())
         padded = tiles * ntok
         ints = torch.empty(Z + (Z + 1) + 2 * rows + padded, dtype=torch.int32, device=dev)
         counts, offs = ints[:Z], ints[Z:2 * Z + 1]

@@ -183,3 +183,35 @@ def test_decode_work_items_remembered_between_steps_are_the_same():
             b = ops.decode_work_items(pos, 4, window, sms=148)
             assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2] == b[2]
         assert batch > 1 or reused >= 140
+
+
+@pytest.mark.parametrize("E,Z", [(1, 1), (1, 16), (3, 5), (8, 8), (64, 64)])
+@pytest.mark.parametrize("T", [1, 16, 17, 32, 33, 100, 700, 5000])
+@pytest.mark.parametrize("top", [1, 2, 16])
+@pytest.mark.parametrize("F", [40, 672, 4096])
+def test_expert_tiles_hold_every_choice(E, Z, T, top, F):
+    """Tiles of the experts' products: steps of up to 32 tokens keep the tiles that their split-K workspace is counted for, no
+    grid passes the limit, and the tiles hold the worst choice there is (as many experts as can be with one row too many)."""
+    if top > Z:
+        return
+    for gated in (True, False):
+        ntok, pair, tiles = ops._expert_tiles(T, top, E, Z, F, gated, 148)
+        assert pair == (2 if ntok == 128 else 1) and ntok // pair == (16 if T <= 16 else 32 if T <= 32 else 64)
+        assert gated or pair == 1
+        rows, worst = T * top, 0
+        for full in range(min(E, rows) + 1):              # `full` experts with a multiple of the tile plus one row
+            left = rows - full
+            if left < 0:
+                break
+            worst = max(worst, full + left // ntok + (1 if left % ntok and full < E else 0))
+        assert min(worst, rows) <= tiles <= 65535 // pair
+
+
+def test_expert_tiles_of_128_rows_only_where_tiles_of_64_wait():
+    """Both sides of the line: one expert's tile column per 64 rows and 128 hidden entries against the SMs, and the largest grid."""
+    tiles = lambda T, top, E, Z, F: ops._expert_tiles(T, top, E, Z, F, True, 148)[0]                   # noqa: E731
+    assert tiles(512, 2, 8, 8, 672) == 64 and tiles(704, 2, 8, 8, 672) == 128        # 120 and 156 CTAs
+    assert tiles(2048, 2, 8, 8, 256) == 64 and tiles(2800, 2, 8, 8, 256) == 128
+    assert tiles(1020, 2, 8, 16, 672) == 64                # half of the choices are identity experts
+    rows = 65535 * 64 - 64 * 256                           # tiles of 64 fit the grid, twice the tiles of 128 would not
+    assert ops._expert_tiles(rows, 1, 256, 256, 4096, True, 148)[:2] == (64, 1)

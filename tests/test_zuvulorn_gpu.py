@@ -560,9 +560,10 @@ def test_experts_on_tensor_cores_against_cuda_cores(T, W, F, E, top):
         assert float((got - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
 
 
-@pytest.mark.parametrize("T, W, F, E, top", [(600, 192, 136, 4, 2), (900, 128, 264, 3, 1), (1030, 72, 128, 8, 2), (256, 64, 40, 1, 1)])
+@pytest.mark.parametrize("T, W, F, E, top", [(600, 192, 136, 4, 2), (900, 128, 264, 3, 1), (1030, 72, 128, 8, 2), (256, 64, 40, 1, 1),
+                                             (600, 192, 1160, 4, 2), (900, 128, 2056, 3, 1), (1030, 72, 1000, 8, 2), (256, 64, 4200, 1, 1)])
 def test_experts_in_tiles_of_128_rows(T, W, F, E, top):
-    """256 rows an expert and more: stretches of several tiles, part-filled ones, an expert without a token, against the
+    """Many rows an expert, in tiles of 64 (few hidden entries) and of 128: stretches of several tiles, part-filled ones, an expert without a token, against the
     CUDA-core kernels on the same choice.  Bound as above (bfloat16 hidden layers)."""
     from prism_b200 import ops
     g = torch.Generator().manual_seed(T + E)
