@@ -22,11 +22,11 @@
 // experts have few tiles).
 //
 // A decode step (a few rows per expert) reads every chosen expert's weights once; a prompt's tiles of one expert
-// re-read them from L2, and that is what bounds them: a k-block of a 128 x 64 tile brings 24 KB for a million
-// multiply-adds' worth of MMA time far below its way from L2.  So the
-// gate and up product takes tiles of 128 rows where the experts have rows enough (brought in boxes of 64, only those that
-// hold rows; the MMA's N is the rows rounded up to 16): 1,999 tokens, 8 experts of 2 x 1,184 x 4,096, 2 identity
-// experts: 147 -> 109 us.  256 rows took 127 us (160 CTAs on 148 SMs), and the down product, with K of 1,184, gains nothing.  Every mbarrier wait is bounded, as in gemm_tcgen05.cu.
+// re-read them from L2, and that is what bounds them: a k-block of a gate and up tile of 64 rows brings 40 KB for a million
+// multiply-adds, MMA time far below its way from L2.  So that product takes tiles of 128 rows (48 KB for two million) where there are
+// tiles enough (brought in boxes of 64, only those that hold rows; the MMA's N is the rows rounded up to 16): 1,999 tokens, 8 experts
+// of 2 x 1,184 x 4,096, 2 identity experts: 147 -> 109 us.  256 rows took 127 us (160 CTAs on 148 SMs), and the down product, with K
+// of 1,184, gains nothing.  Every mbarrier wait is bounded, as in gemm_tcgen05.cu.
 #include "tcgen05.cuh"
 
 #include <type_traits>
@@ -192,15 +192,16 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         pdl_wait();
         const int* row_dst = pdl_fresh(row_dst_in);
         const float* row_w = pdl_fresh(row_w_in);
-        // where the tile's rows go and what they are multiplied by, a row a lane, while the products run (DUAL: not used)
-        constexpr int HOLD = DUAL ? 1 : (NTOK + 31) / 32;
+        // where the tile's rows go and what they are multiplied by, a row a lane, while the products run (few rows only)
+        constexpr bool AHEAD = !DUAL && NTOK < 64;
+        constexpr int HOLD = AHEAD ? (NTOK + 31) / 32 : 1;
         int to[HOLD];
         float by[HOLD];
 #pragma unroll
         for (int k = 0; k < HOLD; ++k) {
             const int n = lane + 32 * k, p = row0 + n;
-            to[k] = !DUAL && !shared_tile && row_dst != nullptr && n < valid ? row_dst[p] : p;
-            by[k] = !DUAL && !shared_tile && row_dst != nullptr && row_w != nullptr && n < valid ? row_w[p] : 1.f;
+            to[k] = AHEAD && !shared_tile && row_dst != nullptr && n < valid ? row_dst[p] : p;
+            by[k] = AHEAD && !shared_tile && row_dst != nullptr && row_w != nullptr && n < valid ? row_w[p] : 1.f;
         }
         if (nkb > 0) mbar_wait(acc_bar, 0, abortp);
         asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -288,7 +289,28 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         }
                 }
             }
-            if (finish) finish_rows(acc, 0, std::integral_constant<int, NTOK>());
+            if constexpr (NTOK < 64) {
+                if (finish) finish_rows(acc, 0, std::integral_constant<int, NTOK>());
+            } else if (finish && m < N) {
+                // full tiles of a prompt: a row at a time (8 experts of 2 x 672 x 2,048, 64 rows each: gate and up 22.5 us, down 30;
+                // eight rows side by side 29 and 38)
+#pragma unroll
+                for (int n = 0; n < NTOK; ++n) {
+                    if (n >= valid) continue;
+                    const int p = row0 + n;
+                    if (shared_tile && !DUAL) {
+                        reinterpret_cast<float*>(y)[(size_t)p * ldy + m] = acc[0][n];
+                    } else if (DUAL) {
+                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] =
+                            __float2bfloat16_rn(moe_tc_glu<CLAMP>(acc[0][n], acc[W_TILES - 1][n], act, limit));
+                    } else if (row_dst == nullptr) {          // an expert without a gate: its hidden layer, act(up a_p)
+                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(moe_tc_act(acc[0][n], act));
+                    } else {
+                        const float v = row_w != nullptr ? acc[0][n] * row_w[p] : acc[0][n];
+                        reinterpret_cast<float*>(y)[(size_t)row_dst[p] * ldy + m] = v;
+                    }
+                }
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
