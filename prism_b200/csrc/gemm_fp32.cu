@@ -139,24 +139,29 @@ few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __
 }
 
 // ---- many rows --------------------------------------------------------------------------------------
-// BM x BN outputs a CTA, TM x TN a thread, one slice of K a step (the next one on its way in registers), the
-// multiply-adds in pairs of rows (fma.rn.f32x2).  SPLIT: the eight classes of a tile are the eight CTAs of a
-// cluster, whose sums meet through distributed shared memory; taken where the tiles alone would not fill the GPU.
-template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC>
+// BM x BN outputs a CTA, TM x TN a thread, a slice of K or half of one a step (the next one on its way in registers), the
+// multiply-adds in pairs of rows (fma.rn.f32x2).  Neighbouring lanes bring the neighbouring bytes of a row, and what they
+// store transposed lies at row ^ TURN (k / 4), so that a warp's stores meet no bank twice and rows stay together in fours.
+// (Lanes that brought a row each took 32 half-used sectors a load: 252 rows, N 9,728, K 896 193 us, now 130; the
+// multiply-adds alone would take 61.  A 128-bit load from shared memory keeps the SM's path to the registers busy for four cycles
+// whatever its lanes share, so the loads weigh nearly as much as the multiply-adds; a second copy of W with its columns swapped
+// instead of the two moves a column took 164 us, 8 x 8 outputs a thread 136: fewer loads, but half the warps to cover them.)
+// SPLIT: the eight classes of a tile are the eight CTAs of a cluster, whose sums meet through distributed shared memory.
+template <int BM, int BN, int STEP, bool SPLIT> constexpr int many_smem() { return (2 * STEP * (BM + BN) + (SPLIT ? BM * BN : 0)) * 4; }
+
+template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
                  int bias_bf16, float* C, int ldc, int M, int N, int K) {
-    constexpr int THREADS = (BM / TM) * (BN / TN);
-    constexpr int LA = BM * 8 / THREADS, LW = BN * 8 / THREADS;      // 16-byte pieces of a slice a thread brings
-    static_assert(BM % 32 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN == 4 && LA * THREADS == BM * 8 && LW * THREADS == BN * 8, "");
-    struct Tiles {
-        float a[2][SLICE][BM];
-        float w[2][SLICE][BN];
-    };
-    __shared__ __align__(16) union {
-        Tiles t;
-        float sums[SPLIT ? BM : 1][SPLIT ? BN : 1];
-    } sm;
+    constexpr int THREADS = (BM / TM) * (BN / TN), OWN = SPLIT ? 1 : CLASSES;       // classes of this CTA
+    constexpr int P = STEP / 4, TURN = 32 / P;                       // 16-byte pieces of a row a step
+    constexpr int LA = BM * P / THREADS, LW = BN * P / THREADS;      // pieces a thread brings
+    static_assert(BM % 32 == 0 && BN % 32 == 0 && TM % 4 == 0 && TN % 4 == 0 && LA * THREADS == BM * P && LW * THREADS == BN * P &&
+                  (STEP == SLICE || STEP == SLICE / 2), "");
+    extern __shared__ __align__(16) float smem[];
+    float* as = smem;                              // [2][STEP][BM]
+    float* ws = smem + 2 * STEP * BM;              // [2][STEP][BN]
+    float* sums = ws + 2 * STEP * BN;              // [BM][BN] of a split tile
     const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int slices = (K + SLICE - 1) / SLICE;
@@ -183,29 +188,30 @@ many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* _
         }
         return v;
     };
-    // neighbouring threads bring neighbouring rows: their transposed stores meet no bank twice
-    auto fetch = [&](int c) {
+    auto fetch = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < LA; ++i) {
             const int idx = tid + i * THREADS;
-            ra[i] = piece(A, lda, m0 + idx % BM, M, c * SLICE + idx / BM * 4);
+            ra[i] = piece(A, lda, m0 + idx / P, M, k0 + idx % P * 4);
         }
 #pragma unroll
         for (int i = 0; i < LW; ++i) {
             const int idx = tid + i * THREADS;
-            rw[i] = piece(W, ldw, n0 + idx % BN, N, c * SLICE + idx / BN * 4);
+            rw[i] = piece(W, ldw, n0 + idx / P, N, k0 + idx % P * 4);
         }
     };
     auto put = [&](int b) {
 #pragma unroll
         for (int i = 0; i < LA; ++i) {
-            const int idx = tid + i * THREADS, r = idx % BM, k = idx / BM * 4;
-            sm.t.a[b][k][r] = ra[i].x, sm.t.a[b][k + 1][r] = ra[i].y, sm.t.a[b][k + 2][r] = ra[i].z, sm.t.a[b][k + 3][r] = ra[i].w;
+            const int idx = tid + i * THREADS, p = idx % P;
+            float* d = as + (b * STEP + 4 * p) * BM + ((idx / P) ^ (TURN * p));
+            d[0] = ra[i].x, d[BM] = ra[i].y, d[2 * BM] = ra[i].z, d[3 * BM] = ra[i].w;
         }
 #pragma unroll
         for (int i = 0; i < LW; ++i) {
-            const int idx = tid + i * THREADS, r = idx % BN, k = idx / BN * 4;
-            sm.t.w[b][k][r] = rw[i].x, sm.t.w[b][k + 1][r] = rw[i].y, sm.t.w[b][k + 2][r] = rw[i].z, sm.t.w[b][k + 3][r] = rw[i].w;
+            const int idx = tid + i * THREADS, p = idx % P;
+            float* d = ws + (b * STEP + 4 * p) * BN + ((idx / P) ^ (TURN * p));
+            d[0] = rw[i].x, d[BN] = rw[i].y, d[2 * BN] = rw[i].z, d[3 * BN] = rw[i].w;
         }
     };
 
@@ -217,13 +223,9 @@ many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* _
         for (int q = 0; q < TN; ++q) acc[i][q] = 0;
     for (auto& t : total)
         for (auto& v : t) v = 0.f;
-    int b = 0, cls = first, c = first;
-    // the slice after c in this CTA's order; the classes of an unsplit tile follow one another
-    auto after = [&](int& cl, int s) {
-        s += CLASSES;
-        while (!SPLIT && s >= slices && ++cl < CLASSES) s = cl;
-        return s;
-    };
+    // row of accumulator i, column of accumulator q (fours lie together)
+    auto row = [&](int i) { return ty * 4 + i / 4 * (BM / (TM / 4)) + i % 4; };
+    auto column = [&](int q) { return tx * 4 + q / 4 * (BN / (TN / 4)) + q % 4; };
     auto close = [&](int cl) {                     // the sums of class cl are complete
         if constexpr (!SPLIT) {
 #pragma unroll
@@ -235,83 +237,105 @@ many_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* _
                     total[2 * i + 1][q] = cl == 0 ? v.y : total[2 * i + 1][q] + v.y;
                     acc[i][q] = 0;
                 }
+        } else {
+#pragma unroll
+            for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+                for (int q = 0; q < TN; q += 4) {
+                    const float2 v[4] = {unpack2(acc[i][q]), unpack2(acc[i][q + 1]), unpack2(acc[i][q + 2]), unpack2(acc[i][q + 3])};
+                    *reinterpret_cast<float4*>(sums + row(2 * i) * BN + column(q)) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+                    *reinterpret_cast<float4*>(sums + row(2 * i + 1) * BN + column(q)) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+                }
         }
     };
+    // The CTA's classes follow one another, a class's slices in ascending order, a slice in one step or two (the second only
+    // where K reaches into it).
+    int cls = first, c = first, h = 0, b = 0;
     if (c < slices) {
-        fetch(c);
+        fetch(c * SLICE);
         put(0);
         __syncthreads();
         while (true) {
-            int ncls = cls;
-            const int nc = after(ncls, c);
+            int ncls = cls, nc = c, nh = 0;
+            if (STEP < SLICE && h == 0 && c * SLICE + STEP < K) {
+                nh = 1;
+            } else {
+                nc += CLASSES;
+                while (nc >= slices && ++ncls < first + OWN) nc = ncls;
+            }
             const bool more = nc < slices;
-            if (more) fetch(nc);
+            if (more) fetch(nc * SLICE + nh * STEP);
 #pragma unroll
-            for (int k = 0; k < SLICE; ++k) {
+            for (int k = 0; k < STEP; ++k) {
+                const float* ak = as + (b * STEP + k) * BM + ((ty * 4) ^ (TURN * (k / 4)));
+                const float* wk = ws + (b * STEP + k) * BN + ((tx * 4) ^ (TURN * (k / 4)));
                 ulonglong2 a[TM / 4];
 #pragma unroll
-                for (int i = 0; i < TM / 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(&sm.t.a[b][k][ty * 4 + i * (BM / (TM / 4))]);
-                const float4 w = *reinterpret_cast<const float4*>(&sm.t.w[b][k][tx * 4]);
-                const uint64_t w2[4] = {pack2(w.x, w.x), pack2(w.y, w.y), pack2(w.z, w.z), pack2(w.w, w.w)};
+                for (int i = 0; i < TM / 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(ak + i * (BM / (TM / 4)));
 #pragma unroll
-                for (int i = 0; i < TM / 4; ++i)
+                for (int q = 0; q < TN; q += 4) {
+                    const float4 w = *reinterpret_cast<const float4*>(wk + q / 4 * (BN / (TN / 4)));
+                    const uint64_t w2[4] = {pack2(w.x, w.x), pack2(w.y, w.y), pack2(w.z, w.z), pack2(w.w, w.w)};
 #pragma unroll
-                    for (int q = 0; q < TN; ++q) {
-                        fma2(acc[2 * i][q], a[i].x, w2[q]);
-                        fma2(acc[2 * i + 1][q], a[i].y, w2[q]);
-                    }
+                    for (int i = 0; i < TM / 4; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            fma2(acc[2 * i][q + e], a[i].x, w2[e]);
+                            fma2(acc[2 * i + 1][q + e], a[i].y, w2[e]);
+                        }
+                }
             }
-            if (!SPLIT && (!more || ncls != cls))
-                for (int cl = cls; cl < (more ? ncls : CLASSES); ++cl) close(cl);      // empty classes add their zero too
+            if (!more || ncls != cls)
+                for (int cl = cls; cl < (more ? ncls : first + OWN); ++cl) close(cl);      // empty classes add their zero too
             if (!more) break;
             put(b ^ 1);
             __syncthreads();
-            b ^= 1, c = nc, cls = ncls;
-        }
-    }
-    // row of accumulator i (pairs lie in groups of four rows)
-    auto row = [&](int i) { return ty * 4 + i / 4 * (BM / (TM / 4)) + i % 4; };
-    if constexpr (!SPLIT) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int m = m0 + row(i);
-            if (m >= M) continue;
-#pragma unroll
-            for (int q = 0; q < TN; ++q) {
-                const int n = n0 + tx * 4 + q;
-                if (n >= N) continue;
-                float v = total[i][q];
-                if (bias != nullptr) v += load_param(bias, bias_bf16, n);
-                C[(size_t)m * ldc + n] = v;
-            }
+            b ^= 1, c = nc, cls = ncls, h = nh;
         }
     } else {
-        __syncthreads();
+        for (int cl = first; cl < first + OWN; ++cl) close(cl);
+    }
+    const bool quads = N % 4 == 0 && ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
+    auto store = [&](int m, int n, float4 v) {
+        if (m >= M || n >= N) return;
+        if (bias != nullptr) {
+            v.x += load_param(bias, bias_bf16, n);
+            if (n + 1 < N) v.y += load_param(bias, bias_bf16, n + 1);
+            if (n + 2 < N) v.z += load_param(bias, bias_bf16, n + 2);
+            if (n + 3 < N) v.w += load_param(bias, bias_bf16, n + 3);
+        }
+        float* d = C + (size_t)m * ldc + n;
+        if (quads) {
+            *reinterpret_cast<float4*>(d) = v;
+        } else {
+            d[0] = v.x;
+            if (n + 1 < N) d[1] = v.y;
+            if (n + 2 < N) d[2] = v.z;
+            if (n + 3 < N) d[3] = v.w;
+        }
+    };
+    if constexpr (!SPLIT) {
 #pragma unroll
-        for (int i = 0; i < TM / 2; ++i)
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int q = 0; q < TN; ++q) {
-                const float2 v = unpack2(acc[i][q]);
-                sm.sums[row(2 * i)][tx * 4 + q] = v.x;
-                sm.sums[row(2 * i + 1)][tx * 4 + q] = v.y;
-            }
+            for (int q = 0; q < TN; q += 4)
+                store(m0 + row(i), n0 + column(q), make_float4(total[i][q], total[i][q + 1], total[i][q + 2], total[i][q + 3]));
+    } else {
         asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
         // this CTA adds up an eighth of the tile's rows
-        for (int idx = tid; idx < BM / CLASSES * BN; idx += THREADS) {
-            const int r = first * (BM / CLASSES) + idx / BN, n = idx % BN;
-            float v = 0.f;
+        for (int idx = tid; idx < BM / CLASSES * (BN / 4); idx += THREADS) {
+            const int r = first * (BM / CLASSES) + idx / (BN / 4), n = idx % (BN / 4) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int cl = 0; cl < CLASSES; ++cl) {
                 uint32_t remote;
-                float x;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&sm.sums[r][n])), "r"(cl));
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
-                v = cl == 0 ? x : v + x;
+                float4 x;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(sums + r * BN + n)), "r"(cl));
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(remote) : "memory");
+                if (cl == 0) v = x;
+                else v.x += x.x, v.y += x.y, v.z += x.z, v.w += x.w;
             }
-            if (m0 + r < M && n0 + n < N) {
-                if (bias != nullptr) v += load_param(bias, bias_bf16, n0 + n);
-                C[(size_t)(m0 + r) * ldc + n0 + n] = v;
-            }
+            store(m0 + r, n0 + n, v);
         }
         asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     }
@@ -353,10 +377,13 @@ template <bool VEC> int few_m(const Call& c) {
     return few_n<16, VEC>(c);
 }
 
-template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC> int many(const Call& c) {
+template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC> int many(const Call& c) {
+    constexpr int smem = many_smem<BM, BN, STEP, SPLIT>();
+    static_assert(smem <= 48 * 1024, "");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((c.N + BN - 1) / BN, (c.M + BM - 1) / BM, SPLIT ? CLASSES : 1);
     cfg.blockDim = dim3((BM / TM) * (BN / TN));
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -365,8 +392,8 @@ template <int BM, int BN, int TM, int TN, bool SPLIT, bool VEC> int many(const C
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, many_rows_kernel<BM, BN, TM, TN, SPLIT, VEC>, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C, c.ldc, c.M,
-                                   c.N, c.K);
+    return (int)cudaLaunchKernelEx(&cfg, many_rows_kernel<BM, BN, TM, TN, STEP, SPLIT, VEC>, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C,
+                                   c.ldc, c.M, c.N, c.K);
 }
 
 template <bool VEC> int pick(const Call& c) {
@@ -378,12 +405,15 @@ template <bool VEC> int pick(const Call& c) {
     int rows = 1;
     while (rows < c.M && rows < 32) rows *= 2;
     if (c.K <= (rows == 32 ? 3 * SLICE : (c.N < 1500 ? 3 : c.N < 4736 ? 10 : 12) * rows))
-        return tiles(32, 32) <= 1500 ? many<32, 32, 4, 4, false, VEC>(c) : many<128, 64, 8, 4, false, VEC>(c);
+        return tiles(32, 32) <= 1500 ? many<32, 32, 4, 4, 32, false, VEC>(c) : many<64, 64, 8, 4, 16, false, VEC>(c);
     if (c.M <= 16) return few_m<VEC>(c);
-    // tiles of 64 x 64 that do not fill the 148 SMs twice have their K shared by a cluster, as far as its CTAs have slices
-    if (tiles(64, 64) * PERIOD < 296LL * (c.K < PERIOD ? c.K : PERIOD)) return many<64, 64, 4, 4, true, VEC>(c);
-    if (c.M <= 64) return many<64, 64, 4, 4, false, VEC>(c);
-    return many<128, 64, 8, 4, false, VEC>(c);
+    // Where tiles of 64 x 64 would not fill the SMs some six times over, a cluster shares their K, as far as its CTAs have slices
+    // (252 rows, N 9,728, K 896, 608 tiles: 130 us, unsplit 137; 512 rows, 1,216 tiles: 250 and 229).  Six of its CTAs fit an SM; where
+    // one round holds all, half tiles may share the SMs more evenly, at some 0.55 of the time each (252 rows, K 4,864: N 896 83 us
+    // against 104; K 896, N 1,152 26.6 and 25.6).
+    if (tiles(64, 64) * PERIOD >= 900LL * (c.K < PERIOD ? c.K : PERIOD)) return many<64, 64, 8, 4, 16, false, VEC>(c);
+    const long long whole = (tiles(64, 64) * CLASSES + 147) / 148, half = (tiles(32, 64) * CLASSES + 147) / 148;
+    return c.M <= 32 || (whole <= 6 && 55 * half < 100 * whole) ? many<32, 64, 4, 4, 16, true, VEC>(c) : many<64, 64, 8, 4, 16, true, VEC>(c);
 }
 
 }  // namespace f32gemm

@@ -189,6 +189,22 @@ def test_sgemm_same_at_every_row_count(N, K, pad):
     assert (rows[:, :N].double() - ref).abs().max() < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
 
 
+@pytest.mark.parametrize("N,K", [(65, 47), (60, 112), (1152, 913), (896, 2064), (1000, 2049)])
+def test_sgemm_at_the_edges_of_its_tiles(N, K):
+    """Tiles of 32 and 64 rows, whole or with their K shared by a cluster, at their first and last rows and columns and where K ends in
+    either half of a slice: the bits of one row alone.  Bound: a chain of K / 8 products, sums of eight, |x w| of about 0.05."""
+    ops = _ops()
+    x, w = _rand((257, K), torch.float32, 16), _rand((N, K), torch.float32, 17, 0.05)
+    one = torch.empty(1, N, dtype=torch.float32, device=DEV)
+    ops.sgemm(x[:1], w, None, one)
+    for M in (257, 256, 65, 64, 33, 32, 31, 17):
+        out = torch.empty(M, N, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[:M], w, None, out)
+        assert torch.equal(out[:1], one), M
+        err = (out.double() - x[:M].double() @ w.double().T).abs().max()
+        assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6, M
+
+
 @pytest.mark.parametrize("M", [1, 3, 16, 40])
 def test_linear_reads_a_weight_that_was_just_written(M):
     """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
