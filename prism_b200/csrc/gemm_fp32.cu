@@ -13,14 +13,16 @@
 // one warp) or eight CTAs (few tiles: a cluster) where one chain per output
 // would leave the GPU idle.
 //
-// Few rows (M <= 16) are bound by the stream of weights: measured at 3 rows,
-// K 896, N 151,936 (545 MB) 2.4 ms with one tile kernel for every M, 0.11 ms here.
+// Few rows (M <= 16) are bound by the stream of weights: measured at 3 rows, K 896, N 151,936 (545 MB) 2.4 ms with one tile
+// kernel for every M, 0.09 ms here.
 #include "f32x2.cuh"
 
 namespace prism {
 namespace f32gemm {
 
 constexpr int SLICE = 32, CLASSES = 8, PERIOD = SLICE * CLASSES;
+constexpr int FEW_WARPS = 8;                  // of a CTA that takes few rows, at most
+constexpr int COLUMNS_STAGES = 5;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -32,18 +34,17 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float* src, int bytes)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// ---- few rows -----------------------------------------------------------------------------------------
-// A CTA owns BN weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared
+// ---- few rows, few columns, a short K ----------------------------------------------------------------------
+// A CTA of two warps owns eight weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared
 // memory stages (cp.async; the weights of the first stages are brought into L2 before the dependency wait: read they are
-// after it, so that they may also be what an earlier kernel of the stream writes).  Thread =
-// (class, column group): the eight classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie
-// at (class, piece ^ class), so that the eight lanes read eight different bank groups.
-// BN 8 where N is small (N 896: 112 CTAs), else 32 with two columns a thread, which halves the reads of A.
-template <int MT, int BN, int CPT, int STAGES, bool VEC>
-__global__ void __launch_bounds__(BN / CPT * CLASSES)
-few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
-                int bias_bf16, float* C, int ldc, int M, int N, int K) {
-    constexpr int THREADS = BN / CPT * CLASSES;
+// after it, so that they may also be what an earlier kernel of the stream writes).  Thread = (class, column): the eight
+// classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie at (class, piece ^ class), so that the eight
+// lanes read eight different bank groups.  Bound by latency: N 896 is 112 CTAs with four periods each.
+template <int MT, bool VEC>
+__global__ void __launch_bounds__(8 * CLASSES)
+few_columns_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
+                   int bias_bf16, float* C, int ldc, int M, int N, int K) {
+    constexpr int BN = 8, STAGES = COLUMNS_STAGES, THREADS = BN * CLASSES;
     constexpr int STAGE = (BN + MT) * PERIOD;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, j = tid % CLASSES, cg = tid / CLASSES;
@@ -85,11 +86,9 @@ few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
-    float acc[MT][CPT];
+    float acc[MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int p = 0; p < CPT; ++p) acc[m][p] = 0.f;
+    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
 
     for (int t = 0; t < periods; ++t) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
@@ -106,33 +105,192 @@ few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int at = j * 8 + (i ^ j);
-            float4 w[CPT];
-#pragma unroll
-            for (int p = 0; p < CPT; ++p) w[p] = ws[(cg + p * (BN / CPT)) * (PERIOD / 4) + at];
+            const float4 w = ws[cg * (PERIOD / 4) + at];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 x = xs[m * (PERIOD / 4) + at];
-#pragma unroll
-                for (int p = 0; p < CPT; ++p) {
-                    acc[m][p] = fmaf(x.x, w[p].x, acc[m][p]);
-                    acc[m][p] = fmaf(x.y, w[p].y, acc[m][p]);
-                    acc[m][p] = fmaf(x.z, w[p].z, acc[m][p]);
-                    acc[m][p] = fmaf(x.w, w[p].w, acc[m][p]);
-                }
+                acc[m] = fmaf(x.x, w.x, acc[m]);
+                acc[m] = fmaf(x.y, w.y, acc[m]);
+                acc[m] = fmaf(x.z, w.z, acc[m]);
+                acc[m] = fmaf(x.w, w.w, acc[m]);
             }
         }
     }
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
+        float v = __shfl_sync(0xffffffffu, acc[m], 0, CLASSES);
 #pragma unroll
-        for (int p = 0; p < CPT; ++p) {
-            float v = __shfl_sync(0xffffffffu, acc[m][p], 0, CLASSES);
+        for (int c = 1; c < CLASSES; ++c) v += __shfl_sync(0xffffffffu, acc[m], c, CLASSES);
+        const int n = n0 + cg;
+        if (m % CLASSES == j && m < M && n < N) {
+            if (bias != nullptr) v += load_param(bias, bias_bf16, n);
+            C[(size_t)m * ldc + n] = v;
+        }
+    }
+}
+
+// all but the newest `stages - 1` groups (2 to 8 stages) have landed
+__device__ __forceinline__ void few_wait(int stages) {
+    switch (stages) {
+        case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 6: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        case 7: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+    }
+}
+
+// ---- few rows -----------------------------------------------------------------------------------------
+// Bound by the stream of weights.  A warp takes 4 CPT columns at a time and walks their K in periods of 256 through a
+// ring of its own (cp.async), straight on into the first periods of its next columns; no warp waits for another.  A CTA has a
+// contiguous share of the columns, even to 4 CPT of them over the SMs, and keeps its rows of A whole in shared memory
+// (XRES; a K too long for that sends them through the rings too).  Lane = (class, column): the eight classes of a column
+// are eight neighbouring lanes.  A row's 16-byte pieces lie at (class, piece ^ class), so that the eight lanes read eight
+// different bank groups.  The weights of the first stages are brought into L2 before the dependency wait; read they are after
+// it, so that they may also be what an earlier kernel of the stream writes.
+template <int MT, int CPT, bool VEC, bool XRES>
+__global__ void __launch_bounds__(FEW_WARPS * 32)
+few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
+                int bias_bf16, float* C, int ldc, int M, int N, int K, int stages) {
+    constexpr int COLS = 4 * CPT, ROWS = COLS + (XRES ? 0 : MT);     // rows of a stage
+    extern __shared__ __align__(16) float smem[];
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, warps = blockDim.x / 32, j = lane % CLASSES, cg = lane / CLASSES;
+    const int m0 = blockIdx.y * MT;
+    const int periods = (K + PERIOD - 1) / PERIOD, mrows = min(MT, M - m0);
+    const int groups = (N + COLS - 1) / COLS;
+    const int g1 = (int)((long long)groups * (blockIdx.x + 1) / gridDim.x);
+    const int g0 = (int)((long long)groups * blockIdx.x / gridDim.x) + warp;     // then every `warps`-th
+    const int mine = g0 < g1 ? (g1 - g0 + warps - 1) / warps : 0;
+    float* ring = smem + (XRES ? (size_t)periods * mrows * PERIOD : 0) + (size_t)warp * stages * ROWS * PERIOD;
+
+    // the 64 pieces of a row's period, two a lane; the place of piece p
+    auto place = [](int p) { return (p / 8) * 8 + ((p % 8) ^ (p / 8)); };
+    const int at0 = place(lane) * 4, at1 = place(lane + 32) * 4;
+    auto bring = [&](const float* row, int k, bool live, uint32_t d) {
+        const int have = live ? min(max(K - k, 0), 4) : 0;
+        const float* s = have ? row + k : row;
+        if (VEC) {
+            copy16(d, s, have * 4);
+        } else {
 #pragma unroll
-            for (int c = 1; c < CLASSES; ++c) v += __shfl_sync(0xffffffffu, acc[m][p], c, CLASSES);
-            const int n = n0 + cg + p * (BN / CPT);
-            if ((m * CPT + p) % CLASSES == j && m < M && n < N) {
-                if (bias != nullptr) v += load_param(bias, bias_bf16, n);
-                C[(size_t)m * ldc + n] = v;
+            for (int e = 0; e < 4; ++e) copy4(d + 4 * e, e < have ? s + e : row, e < have ? 4 : 0);
+        }
+    };
+    auto bring_row = [&](const float* row, int k, bool live, float* dst) {
+        bring(row, k + lane * 4, live, smem_addr(dst + at0));
+        bring(row, k + (lane + 32) * 4, live, smem_addr(dst + at1));
+    };
+    int lg = g0, lt = 0, ls = 0, left = mine * periods;       // the next period to ask for and the stage it goes to
+    auto ask = [&]() {
+        if (left > 0) {
+            float* dst = ring + (size_t)ls * ROWS * PERIOD;
+            const int k = lt * PERIOD;
+            if (VEC && k + PERIOD <= K && (lg + 1) * COLS <= N) {
+                const float* s = W + (size_t)lg * COLS * ldw + k + lane * 4;
+                const uint32_t d0 = smem_addr(dst + at0), d1 = smem_addr(dst + at1);
+#pragma unroll
+                for (int c = 0; c < COLS; ++c, s += ldw) {
+                    copy16(d0 + c * PERIOD * 4, s, 16);
+                    copy16(d1 + c * PERIOD * 4, s + 128, 16);
+                }
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < COLS; ++c) {
+                    const int n = lg * COLS + c;
+                    bring_row(W + (size_t)min(n, N - 1) * ldw, k, n < N, dst + c * PERIOD);
+                }
+            }
+            if (!XRES) {
+#pragma unroll 1
+                for (int m = 0; m < mrows; ++m) bring_row(A + (size_t)(m0 + m) * lda, k, true, dst + (COLS + m) * PERIOD);
+            }
+            if (++lt == periods) lt = 0, lg += warps;
+            if (++ls == stages) ls = 0;
+            --left;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    pdl_trigger();
+    // lines of 128 bytes: eight of a row a period
+    for (int idx = lane; idx < COLS * 8 * stages; idx += 32) {
+        const int n = g0 * COLS + idx % COLS, k = idx / COLS * 32;
+        if (mine && n < N && k < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)n * ldw + k));
+    }
+    pdl_wait();
+    W = pdl_fresh(W), A = pdl_fresh(A);
+    if (XRES) {                                       // lands with the first stage's group
+        for (int idx = warp; idx < periods * mrows; idx += warps) {
+            const int t = idx / mrows, m = idx - t * mrows;
+            bring_row(A + (size_t)(m0 + m) * lda, t * PERIOD, true, smem + (size_t)idx * PERIOD);
+        }
+    }
+    for (int s = 0; s < stages; ++s) ask();
+    if (XRES) {
+        few_wait(stages);
+        __syncthreads();
+    }
+
+    int stage = 0;
+    for (int g = g0; g < g1; g += warps) {
+        float acc[MT][CPT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) acc[m][p] = 0.f;
+        for (int t = 0; t < periods; ++t) {
+            few_wait(stages);
+            __syncwarp();
+            const float4* ws = reinterpret_cast<const float4*>(ring + (size_t)stage * ROWS * PERIOD);
+            const float4* xs = XRES ? reinterpret_cast<const float4*>(smem + (size_t)t * mrows * PERIOD) : ws + COLS * (PERIOD / 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int at = j * 8 + (i ^ j);
+                float4 w[CPT];
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) w[p] = ws[(cg + 4 * p) * (PERIOD / 4) + at];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float4 x = xs[(MT <= 4 ? m : min(m, mrows - 1)) * (PERIOD / 4) + at];
+#pragma unroll
+                    for (int p = 0; p < CPT; ++p) {
+                        acc[m][p] = fmaf(x.x, w[p].x, acc[m][p]);
+                        acc[m][p] = fmaf(x.y, w[p].y, acc[m][p]);
+                        acc[m][p] = fmaf(x.z, w[p].z, acc[m][p]);
+                        acc[m][p] = fmaf(x.w, w[p].w, acc[m][p]);
+                    }
+                }
+            }
+            __syncwarp();
+            ask();                                    // into the stage that was just read
+            if (++stage == stages) stage = 0;
+        }
+        // the classes' sums in ascending order; eight outputs at a time, lane j of a column ends with output j
+        constexpr int OUT = MT * CPT;
+#pragma unroll
+        for (int o0 = 0; o0 < OUT; o0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) v[o] = o0 + o < OUT ? acc[(o0 + o < OUT ? o0 + o : 0) / CPT][(o0 + o) % CPT] : 0.f;
+#pragma unroll
+            for (int s = 4; s; s /= 2)
+#pragma unroll
+                for (int o = 0; o < 8; ++o)
+                    if (!(o & s)) {
+                        const bool up = j & s;
+                        const float got = __shfl_xor_sync(0xffffffffu, up ? v[o] : v[o | s], s);
+                        if (up) v[o] = got;
+                        else v[o | s] = got;
+                    }
+            float sum = v[0];
+#pragma unroll
+            for (int c = 1; c < CLASSES; ++c) sum += v[c];
+            const int o = o0 + j, m = o / CPT, n = g * COLS + cg + 4 * (o % CPT);
+            if (o < OUT && m < mrows && n < N) {
+                if (bias != nullptr) sum += load_param(bias, bias_bf16, n);
+                C[(size_t)(m0 + m) * ldc + n] = sum;
             }
         }
     }
@@ -353,28 +511,69 @@ struct Call {
     cudaStream_t stream;
 };
 
-template <int MT, int BN, int CPT, int STAGES, bool VEC> int few(const Call& c) {
-    constexpr int smem = STAGES * (BN + MT) * PERIOD * 4;
-    auto kern = few_rows_kernel<MT, BN, CPT, STAGES, VEC>;
+template <int MT, bool VEC> int few_columns(const Call& c) {
+    constexpr int smem = COLUMNS_STAGES * (8 + MT) * PERIOD * 4;
+    auto kern = few_columns_kernel<MT, VEC>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
     }
-    return (int)launch_kernel(kern, dim3((c.N + BN - 1) / BN), dim3(BN / CPT * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
-                              c.bb, c.C, c.ldc, c.M, c.N, c.K);
+    return (int)launch_kernel(kern, dim3((c.N + 7) / 8), dim3(8 * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C, c.ldc,
+                              c.M, c.N, c.K);
 }
 
-// BN 8 keeps every SM busy down to N of about a thousand; from 148 x 32 columns on wider CTAs fill the GPU too
-template <int MT, bool VEC> int few_n(const Call& c) {
-    return c.N >= 4736 ? few<MT, 32, 2, 3, VEC>(c) : few<MT, 8, 1, 5, VEC>(c);
+// Shared memory of a CTA: as much as leaves room for the next launch's, or up to what there is
+constexpr int FEW_SMEM = 110 * 1024, FEW_SMEM_MOST = 226 * 1024, FEW_X_MOST = 160 * 1024;
+
+// MT rows a CTA, 4 CPT columns a warp
+template <int MT, int CPT, bool VEC, bool XRES> int few(const Call& c) {
+    const int groups = (c.N + 4 * CPT - 1) / (4 * CPT), periods = (c.K + PERIOD - 1) / PERIOD, blocks = (c.M + MT - 1) / MT;
+    const int x = XRES ? periods * min(c.M, MT) * PERIOD * 4 : 0, per_warp = (4 * CPT + (XRES ? 0 : MT)) * PERIOD * 4;
+    // as many warps as share a CTA's columns evenly
+    const int most = min(FEW_WARPS, (FEW_SMEM_MOST - x) / (2 * per_warp)), each = max(2, (groups + 147) / 148), rounds = (each + most - 1) / most;
+    const int warps = (each + rounds - 1) / rounds;
+    const int ctas = min(148, (groups + warps - 1) / warps);
+    const int stages = max(2, min(8, (FEW_SMEM - x) / (per_warp * warps))), smem = x + stages * per_warp * warps;
+    auto kern = few_rows_kernel<MT, CPT, VEC, XRES>;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return (int)launch_kernel(kern, dim3(ctas, blocks), dim3(warps * 32), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
+                              c.bb, c.C, c.ldc, c.M, c.N, c.K, stages);
+}
+
+// Every column of a thread makes its reads of A serve more products (3 rows, N 151,936: 128 us with one, 93 with two, 89 with four;
+// the kernel before it, 32 columns a CTA, took 123), but few columns want the warps (N 896, K 4,864: 14.3, 18.4, 21.0; before 20.6).
+// Rows by sixteen want the registers (N 151,936: 191 us with two, 287 with four; before 417).
+template <int MT, bool VEC> int few_k(const Call& c) {
+    const long long row = (long long)((c.K + PERIOD - 1) / PERIOD) * PERIOD * 4;       // bytes of a row of A in shared memory
+    if (min(c.M, MT) * row > FEW_X_MOST) {
+        if constexpr (MT > 1) return few_k<MT / 2, VEC>(c);
+        else return few<1, 1, VEC, false>(c);
+    }
+    // four warps a CTA have to fit beside its rows of A
+    const long long room = (FEW_SMEM_MOST - min(c.M, MT) * row) / (4 * 2 * 4 * PERIOD * 4);
+    if constexpr (MT <= 8) {
+        if (c.N >= 148 * 64 && room >= 4) return few<MT, 4, VEC, true>(c);
+        if ((c.N < 148 * 32 && c.M <= 8) || room < 2) return few<MT, 1, VEC, true>(c);
+    }
+    return few<MT, 2, VEC, true>(c);
 }
 
 template <bool VEC> int few_m(const Call& c) {
-    if (c.M <= 1) return few_n<1, VEC>(c);
-    if (c.M <= 2) return few_n<2, VEC>(c);
-    if (c.M <= 4) return few_n<4, VEC>(c);
-    if (c.M <= 8) return few_n<8, VEC>(c);
-    return few_n<16, VEC>(c);
+    // Few columns: their two warps at a time share the copies, which is worth more where K is short, there are one or two rows or
+    // the copies are single entries (K 896, N 896: 1 row 3.6 us, 4.1 by a ring a warp, 3 rows 5.4 and 4.9, 8 rows 6.5 and 7.4; K 4,864:
+    // 1 row 12.5 and 10.0, 3 rows 20.6 and 14.3).
+    if (c.N < 148 * 32 && !(VEC && (c.M <= 2 ? c.M == 1 && c.K >= 2048 && c.N >= 592 : c.K >= (c.M <= 4 ? 640 : 2048))))
+        return c.M <= 1 ? few_columns<1, VEC>(c) : c.M <= 2 ? few_columns<2, VEC>(c) : c.M <= 4 ? few_columns<4, VEC>(c) : c.M <= 8 ?
+               few_columns<8, VEC>(c) : few_columns<16, VEC>(c);
+    if (c.M <= 1) return few_k<1, VEC>(c);
+    if (c.M <= 2) return few_k<2, VEC>(c);
+    if (c.M <= 3) return few_k<3, VEC>(c);
+    if (c.M <= 4) return few_k<4, VEC>(c);
+    if (c.M <= 8) return few_k<8, VEC>(c);
+    return few_k<16, VEC>(c);
 }
 
 template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC> int many(const Call& c) {

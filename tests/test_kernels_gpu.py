@@ -205,6 +205,22 @@ def test_sgemm_at_the_edges_of_its_tiles(N, K):
         assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6, M
 
 
+@pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9475, 900), (4800, 5200), (600, 41216), (33, 41217)])
+def test_sgemm_of_few_rows_with_long_rings(N, K):
+    """Few rows: columns that do not fill a warp's or a CTA's share, a ring that runs on into the next columns, rows of x that fit beside
+    it by sixteen, eight, four or one, or not at all: the bits of the tiles.  Bound: as above."""
+    ops = _ops()
+    x, w = _rand((64, K), torch.float32, 18), _rand((N, K), torch.float32, 19, 0.05)
+    tiles = torch.empty(64, N, dtype=torch.float32, device=DEV)
+    ops.sgemm(x, w, None, tiles)
+    err = (tiles[:16].double() - x[:16].double() @ w.double().T).abs().max()
+    assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
+    for M in (16, 13, 9, 8, 5, 4, 3, 2, 1):
+        out = torch.empty(M, N, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[:M], w, None, out)
+        assert torch.equal(out, tiles[:M]), M
+
+
 @pytest.mark.parametrize("M", [1, 3, 16, 40])
 def test_linear_reads_a_weight_that_was_just_written(M):
     """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
