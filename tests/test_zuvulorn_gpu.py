@@ -268,6 +268,28 @@ def test_second_halves_of_the_low_rank_products_with_their_epilogues(T, R, H, pe
     assert float((out.cpu() - torch.sigmoid(z)).abs().max()) <= 3e-6
 
 
+@pytest.mark.parametrize("T", [1, 8, 9, 16])
+@pytest.mark.parametrize("blocks, bs, R", [(3, 128, 64), (2, 136, 17), (1, 72, 16), (2, 300, 33), (2, 66, 15)])
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+def test_gates_and_low_rank_products_of_few_tokens(T, blocks, bs, R, wdt):
+    """The kernels of up to sixteen (eight) tokens, one round of 128 k and more, in 16-byte pieces and entry by entry: every sum has the
+    order of the kernels of many tokens, so the bits are theirs."""
+    from prism_b200 import ops
+    g = torch.Generator().manual_seed(bs + T)
+    n = lambda *s: torch.randn(*s, generator=g).to(DEV)                                   # noqa: E731
+    C = blocks * bs
+    u, low = n(40, C), n(40, R)
+    wr, wi, br, bi, lam = [t.to(wdt) for t in (n(blocks, bs, bs) / bs ** 0.5, n(blocks, bs, bs) / bs ** 0.5, n(C), n(C), n(C) - 2.0)]
+    w2t, b = n(R, C) / R ** 0.5, n(C).to(wdt)
+    many, few = torch.empty(2, 40, C, device=DEV), torch.full((2, T + 1, C), 7.0, device=DEV)
+    ops.block_gates(u, wr, wi, br, bi, lam, 8.0, many[0], many[1])
+    ops.block_gates(u[:T], wr, wi, br, bi, lam, 8.0, few[0, :T], few[1, :T])
+    assert torch.equal(few[:, :T], many[:, :T]) and bool((few[:, T] == 7.0).all())
+    ops.lowrank_decay(low, w2t, b, many[0])
+    ops.lowrank_decay(low[:T], w2t, b, few[0, :T])
+    assert torch.equal(few[0, :T], many[0, :T]) and bool((few[0, T] == 7.0).all())
+
+
 @pytest.mark.parametrize("G, H, dk, dv, K", [(1, 2, 8, 16, 4), (2, 4, 6, 5, 3), (1, 1, 1, 1, 1), (1, 3, 3, 2, 6)])
 def test_convolutions_of_q_k_v_unit_vectors_and_beta(G, H, dk, dv, K):
     from prism_b200 import ops
