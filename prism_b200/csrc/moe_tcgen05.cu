@@ -192,8 +192,8 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         pdl_wait();
         const int* row_dst = pdl_fresh(row_dst_in);
         const float* row_w = pdl_fresh(row_w_in);
-        // where the tile's rows go and what they are multiplied by, a row a lane, while the products run (few rows only)
-        constexpr bool AHEAD = !DUAL && NTOK < 64;
+        // where the tile's rows go and what they are multiplied by, a row a lane, while the products run
+        constexpr bool AHEAD = !DUAL;
         constexpr int HOLD = AHEAD ? (NTOK + 31) / 32 : 1;
         int to[HOLD];
         float by[HOLD];
@@ -228,21 +228,26 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     if (DUAL || (!shared_tile && row_dst == nullptr)) {       // a hidden layer; without a gate act(up a_p)
                         if (live) reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(v[j]);
                     } else {
-                        const int dst = __shfl_sync(0xffffffffu, to[(j0 + j) / 32 % HOLD], (j0 + j) % 32);
-                        const float wt = __shfl_sync(0xffffffffu, by[(j0 + j) / 32 % HOLD], (j0 + j) % 32);
+                        const int dst = __shfl_sync(0xffffffffu, HOLD > 1 && n0 >= 32 ? to[HOLD - 1] : to[0], n0 % 32 + j0 + j);
+                        const float wt = __shfl_sync(0xffffffffu, HOLD > 1 && n0 >= 32 ? by[HOLD - 1] : by[0], n0 % 32 + j0 + j);
                         if (live) reinterpret_cast<float*>(y)[(size_t)dst * ldy + m] = v[j] * wt;
                     }
                 }
             }
         };
-        if constexpr (NTOK > 64) {                       // K is never split here
+        if constexpr (NTOK >= 64) {                      // K is never split here
+            // Sixteen rows at a time in a loop that stays a loop: a CTA runs its epilogue once, and all rows in straight line code are
+            // some 60 KB of instructions that it first has to fetch.  8 experts, all rows unrolled and now: 2 x 672 x 2,048, 256 tokens 72 ->
+            // 58 us, 2,048 154 -> 125; 896 x 2,048 without a gate, 64 tokens 45 -> 32, 2,048 153 -> 106; 32 rows at a time 63, 130, 33, 110.
+            constexpr int PART = 16;
             if (go && nkb > 0)
-                for (int n0 = 0; n0 < valid; n0 += 32) {
-                    float acc[W_TILES][32];
+#pragma unroll 1
+                for (int n0 = 0; n0 < valid; n0 += PART) {
+                    float acc[W_TILES][PART];
 #pragma unroll
                     for (int w = 0; w < W_TILES; ++w)
-                        tmem_load<32>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + n0, acc[w]);
-                    finish_rows(acc, n0, std::integral_constant<int, 32>());
+                        tmem_load<PART>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + n0, acc[w]);
+                    finish_rows(acc, n0, std::integral_constant<int, PART>());
                 }
         } else if (go) {
             float acc[W_TILES][NTOK];
@@ -289,28 +294,7 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         }
                 }
             }
-            if constexpr (NTOK < 64) {
-                if (finish) finish_rows(acc, 0, std::integral_constant<int, NTOK>());
-            } else if (finish && m < N) {
-                // full tiles of a prompt: a row at a time (8 experts of 2 x 672 x 2,048, 64 rows each: gate and up 22.5 us, down 30;
-                // eight rows side by side 29 and 38)
-#pragma unroll
-                for (int n = 0; n < NTOK; ++n) {
-                    if (n >= valid) continue;
-                    const int p = row0 + n;
-                    if (shared_tile && !DUAL) {
-                        reinterpret_cast<float*>(y)[(size_t)p * ldy + m] = acc[0][n];
-                    } else if (DUAL) {
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] =
-                            __float2bfloat16_rn(moe_tc_glu<CLAMP>(acc[0][n], acc[W_TILES - 1][n], act, limit));
-                    } else if (row_dst == nullptr) {          // an expert without a gate: its hidden layer, act(up a_p)
-                        reinterpret_cast<__nv_bfloat16*>(y)[(size_t)p * ldy + m] = __float2bfloat16_rn(moe_tc_act(acc[0][n], act));
-                    } else {
-                        const float v = row_w != nullptr ? acc[0][n] * row_w[p] : acc[0][n];
-                        reinterpret_cast<float*>(y)[(size_t)row_dst[p] * ldy + m] = v;
-                    }
-                }
-            }
+            if (finish) finish_rows(acc, 0, std::integral_constant<int, NTOK>());
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -423,7 +407,7 @@ PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void
     if (E < 1 || K < 8 || K % 8 || lda % 8 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || token_tiles > 65535 ||
         (ntok != 16 && ntok != 32 && ntok != 64 && !(ntok == 128 && dual)))
         return (int)cudaErrorInvalidValue;
-    if (ksplit < 1 || ksplit > (ntok > 64 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
+    if (ksplit < 1 || ksplit > (ntok >= 64 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
     if (shared_rows > 0 && (sw == nullptr || sx == nullptr || sy == nullptr || sN < 1 || sK < 8 || sK % 8 || ldsx % 8 ||
                             ((uintptr_t)sw & 15) || ((uintptr_t)sx & 15) || (!dual && row_dst == nullptr)))
         return (int)cudaErrorInvalidValue;
