@@ -235,7 +235,7 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
             }
         };
-        if constexpr (NTOK >= 64) {                      // K is never split here
+        if constexpr (NTOK >= 32) {                      // K is never split here
             // Sixteen rows at a time in a loop that stays a loop: a CTA runs its epilogue once, and all rows in straight line code are
             // some 60 KB of instructions that it first has to fetch.  8 experts, all rows unrolled and now: 2 x 672 x 2,048, 256 tokens 72 ->
             // 58 us, 2,048 154 -> 125; 896 x 2,048 without a gate, 64 tokens 45 -> 32, 2,048 153 -> 106; 32 rows at a time 63, 130, 33, 110.
@@ -407,7 +407,7 @@ PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void
     if (E < 1 || K < 8 || K % 8 || lda % 8 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || token_tiles > 65535 ||
         (ntok != 16 && ntok != 32 && ntok != 64 && !(ntok == 128 && dual)))
         return (int)cudaErrorInvalidValue;
-    if (ksplit < 1 || ksplit > (ntok >= 64 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
+    if (ksplit < 1 || ksplit > (ntok >= 32 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
     if (shared_rows > 0 && (sw == nullptr || sx == nullptr || sy == nullptr || sN < 1 || sK < 8 || sK % 8 || ldsx % 8 ||
                             ((uintptr_t)sw & 15) || ((uintptr_t)sx & 15) || (!dual && row_dst == nullptr)))
         return (int)cudaErrorInvalidValue;
