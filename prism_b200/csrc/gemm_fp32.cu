@@ -535,10 +535,9 @@ template <int MT, int CPT, bool VEC, bool XRES> int few(const Call& c) {
     const int ctas = min(148, (groups + warps - 1) / warps);
     const int stages = max(2, min(8, (FEW_SMEM - x) / (per_warp * warps))), smem = x + stages * per_warp * warps;
     auto kern = few_rows_kernel<MT, CPT, VEC, XRES>;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-    }
+    // the limit belongs to the function, not to the call: one value, so that no thread's call lowers it under another's
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM_MOST);
+    if (e != cudaSuccess) return (int)e;
     return (int)launch_kernel(kern, dim3(ctas, blocks), dim3(warps * 32), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
                               c.bb, c.C, c.ldc, c.M, c.N, c.K, stages);
 }

@@ -1236,7 +1236,8 @@ PRISM_EXPORT int prism_lowrank_decay(const float* low, long long low_stride, int
     const size_t smem = (size_t)tok * R * sizeof(float);
     if (R < 1 || (size_t)16 * R * sizeof(float) > 200 * 1024 || token_tiles > 65535) return (int)cudaErrorInvalidValue;
     auto kern = tok == 8 ? prism::lowrank_decay_kernel<8> : prism::lowrank_decay_kernel<16>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the function, not to the call: one value, so that no thread's call lowers it under another's
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     return (int)prism::launch_kernel(kern, dim3((N + 127) / 128, token_tiles), dim3(128), smem,
                                      stream, low, low_stride, R, w2t, w0, w0_dtype == PRISM_DTYPE_BF16, N, T, out, out_stride, inner, epi, alog,
                                      alog_dtype == PRISM_DTYPE_BF16, per < 1 ? 1 : per, crate);

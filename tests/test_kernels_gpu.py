@@ -221,6 +221,40 @@ def test_sgemm_of_few_rows_with_long_rings(N, K):
         assert torch.equal(out, tiles[:M]), M
 
 
+def test_calls_of_several_threads_do_not_change_each_others_limits():
+    """Kernels whose shared memory depends on the sizes of the call: the limit belongs to the kernel, so a thread's small call must not
+    lower it between another's setting and its launch."""
+    import threading
+    ops = _ops()
+    errors = []
+
+    def products(K):
+        x, w = _rand((3, K), torch.float32, 21), _rand((896, K), torch.float32, 22)
+        out = torch.empty(3, 896, dtype=torch.float32, device=DEV)
+        return lambda: ops.sgemm(x, w, None, out)
+
+    def decays(R):
+        low, w2t = _rand((4, R), torch.float32, 23), _rand((R, 128), torch.float32, 24)
+        out = torch.empty(4, 128, dtype=torch.float32, device=DEV)
+        return lambda: ops.lowrank_decay(low, w2t, None, out)
+
+    def many(call):
+        try:
+            for _ in range(3000):
+                call()
+        except ops.KernelError as e:
+            errors.append(e)
+
+    for make, sizes in ((products, (896, 13568)), (decays, (1600, 3200))):
+        threads = [threading.Thread(target=many, args=(make(n),)) for n in sizes * 2]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert not errors, (make.__name__, errors[0])
+
+
 @pytest.mark.parametrize("M", [1, 3, 16, 40])
 def test_linear_reads_a_weight_that_was_just_written(M):
     """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
