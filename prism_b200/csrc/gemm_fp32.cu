@@ -22,7 +22,6 @@ namespace f32gemm {
 
 constexpr int SLICE = 32, CLASSES = 8, PERIOD = SLICE * CLASSES;
 constexpr int FEW_WARPS = 8;                  // of a CTA that takes few rows, at most
-constexpr int COLUMNS_STAGES = 5;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -34,17 +33,19 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float* src, int bytes)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// ---- few rows, few columns, a short K ----------------------------------------------------------------------
-// A CTA of two warps owns eight weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared
-// memory stages (cp.async; the weights of the first stages are brought into L2 before the dependency wait: read they are
-// after it, so that they may also be what an earlier kernel of the stream writes).  Thread = (class, column): the eight
-// classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie at (class, piece ^ class), so that the eight
-// lanes read eight different bank groups.  Bound by latency: N 896 is 112 CTAs with four periods each.
-template <int MT, bool VEC>
-__global__ void __launch_bounds__(8 * CLASSES)
-few_columns_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
+// ---- few rows, a ring a CTA ------------------------------------------------------------------------------
+// A CTA owns BN weight rows and all M <= MT rows of A and walks K in periods of 256 through a ring of shared memory stages that both
+// go through, so that W is read once at any K (cp.async; the weights of the first stages are brought into L2 before the dependency
+// wait: read they are after it, so that they may also be what an earlier kernel of the stream writes).  Thread =
+// (class, column group): the eight classes of a column are eight neighbouring lanes.  A row's 16-byte pieces lie
+// at (class, piece ^ class), so that the eight lanes read eight different bank groups.
+// BN 8 where N is small (bound by latency: N 896 is 112 CTAs of two warps), else 32 with two columns a thread, which halves the
+// reads of A.
+template <int MT, int BN, int CPT, int STAGES, bool VEC>
+__global__ void __launch_bounds__(BN / CPT * CLASSES)
+shared_ring_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
                    int bias_bf16, float* C, int ldc, int M, int N, int K) {
-    constexpr int BN = 8, STAGES = COLUMNS_STAGES, THREADS = BN * CLASSES;
+    constexpr int THREADS = BN / CPT * CLASSES;
     constexpr int STAGE = (BN + MT) * PERIOD;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, j = tid % CLASSES, cg = tid / CLASSES;
@@ -86,9 +87,11 @@ few_columns_kernel(const float* A, int lda, const float* W, int ldw, const void*
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
-    float acc[MT];
+    float acc[MT][CPT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int p = 0; p < CPT; ++p) acc[m][p] = 0.f;
 
     for (int t = 0; t < periods; ++t) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
@@ -105,26 +108,34 @@ few_columns_kernel(const float* A, int lda, const float* W, int ldw, const void*
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int at = j * 8 + (i ^ j);
-            const float4 w = ws[cg * (PERIOD / 4) + at];
+            float4 w[CPT];
+#pragma unroll
+            for (int p = 0; p < CPT; ++p) w[p] = ws[(cg + p * (BN / CPT)) * (PERIOD / 4) + at];
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 x = xs[m * (PERIOD / 4) + at];
-                acc[m] = fmaf(x.x, w.x, acc[m]);
-                acc[m] = fmaf(x.y, w.y, acc[m]);
-                acc[m] = fmaf(x.z, w.z, acc[m]);
-                acc[m] = fmaf(x.w, w.w, acc[m]);
+#pragma unroll
+                for (int p = 0; p < CPT; ++p) {
+                    acc[m][p] = fmaf(x.x, w[p].x, acc[m][p]);
+                    acc[m][p] = fmaf(x.y, w[p].y, acc[m][p]);
+                    acc[m][p] = fmaf(x.z, w[p].z, acc[m][p]);
+                    acc[m][p] = fmaf(x.w, w[p].w, acc[m][p]);
+                }
             }
         }
     }
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
-        float v = __shfl_sync(0xffffffffu, acc[m], 0, CLASSES);
 #pragma unroll
-        for (int c = 1; c < CLASSES; ++c) v += __shfl_sync(0xffffffffu, acc[m], c, CLASSES);
-        const int n = n0 + cg;
-        if (m % CLASSES == j && m < M && n < N) {
-            if (bias != nullptr) v += load_param(bias, bias_bf16, n);
-            C[(size_t)m * ldc + n] = v;
+        for (int p = 0; p < CPT; ++p) {
+            float v = __shfl_sync(0xffffffffu, acc[m][p], 0, CLASSES);
+#pragma unroll
+            for (int c = 1; c < CLASSES; ++c) v += __shfl_sync(0xffffffffu, acc[m][p], c, CLASSES);
+            const int n = n0 + cg + p * (BN / CPT);
+            if ((m * CPT + p) % CLASSES == j && m < M && n < N) {
+                if (bias != nullptr) v += load_param(bias, bias_bf16, n);
+                C[(size_t)m * ldc + n] = v;
+            }
         }
     }
 }
@@ -149,9 +160,10 @@ __device__ __forceinline__ void few_wait(int stages) {
 // (XRES; a K too long for that sends them through the rings too).  Lane = (class, column): the eight classes of a column
 // are eight neighbouring lanes.  A row's 16-byte pieces lie at (class, piece ^ class), so that the eight lanes read eight
 // different bank groups.  The weights of the first stages are brought into L2 before the dependency wait; read they are after
-// it, so that they may also be what an earlier kernel of the stream writes.
+// it, so that they may also be what an earlier kernel of the stream writes.  (One CTA an SM by its shared memory: told so, the compiler takes 69
+// to 255 registers; left alone it kept to 64 and spilled, three rows of K 4,864 to N 896 15.8 us against 13.9.)
 template <int MT, int CPT, bool VEC, bool XRES>
-__global__ void __launch_bounds__(FEW_WARPS * 32)
+__global__ void __launch_bounds__(FEW_WARPS * 32, 1)
 few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
                 int bias_bf16, float* C, int ldc, int M, int N, int K, int stages) {
     constexpr int COLS = 4 * CPT, ROWS = COLS + (XRES ? 0 : MT);     // rows of a stage
@@ -511,29 +523,32 @@ struct Call {
     cudaStream_t stream;
 };
 
-template <int MT, bool VEC> int few_columns(const Call& c) {
-    constexpr int smem = COLUMNS_STAGES * (8 + MT) * PERIOD * 4;
-    auto kern = few_columns_kernel<MT, VEC>;
+template <int MT, int BN, int CPT, int STAGES, bool VEC> int shared_ring(const Call& c) {
+    constexpr int smem = STAGES * (BN + MT) * PERIOD * 4;
+    auto kern = shared_ring_kernel<MT, BN, CPT, STAGES, VEC>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
     }
-    return (int)launch_kernel(kern, dim3((c.N + 7) / 8), dim3(8 * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C, c.ldc,
-                              c.M, c.N, c.K);
+    return (int)launch_kernel(kern, dim3((c.N + BN - 1) / BN), dim3(BN / CPT * CLASSES), smem, c.stream, c.A, c.lda, c.W, c.ldw, c.bias,
+                              c.bb, c.C, c.ldc, c.M, c.N, c.K);
 }
 
-// Shared memory of a CTA: as much as leaves room for the next launch's, or up to what there is
-constexpr int FEW_SMEM = 110 * 1024, FEW_SMEM_MOST = 226 * 1024, FEW_X_MOST = 160 * 1024;
+// Shared memory of a CTA: what its rings may take while the rows of A leave room (110 KB instead, for a second CTA, is 4 to 8 % slower on
+// average over 2,400 shapes: two stages where three fit), the same where those rows go through the rings, where two
+// CTAs are to share an SM, and what there is
+constexpr int FEW_SMEM = 160 * 1024, FEW_SMEM_THROUGH = 220 * 1024, FEW_SMEM_TWO = 110 * 1024, FEW_SMEM_MOST = 226 * 1024;
+constexpr int FEW_X_MOST = 160 * 1024;         // rows of A that are kept whole, in bytes
 
 // MT rows a CTA, 4 CPT columns a warp
-template <int MT, int CPT, bool VEC, bool XRES> int few(const Call& c) {
+template <int MT, int CPT, bool VEC, bool XRES> int few(const Call& c, int budget = XRES ? FEW_SMEM : FEW_SMEM_THROUGH) {
     const int groups = (c.N + 4 * CPT - 1) / (4 * CPT), periods = (c.K + PERIOD - 1) / PERIOD, blocks = (c.M + MT - 1) / MT;
     const int x = XRES ? periods * min(c.M, MT) * PERIOD * 4 : 0, per_warp = (4 * CPT + (XRES ? 0 : MT)) * PERIOD * 4;
     // as many warps as share a CTA's columns evenly
     const int most = min(FEW_WARPS, (FEW_SMEM_MOST - x) / (2 * per_warp)), each = max(2, (groups + 147) / 148), rounds = (each + most - 1) / most;
     const int warps = (each + rounds - 1) / rounds;
     const int ctas = min(148, (groups + warps - 1) / warps);
-    const int stages = max(2, min(8, (FEW_SMEM - x) / (per_warp * warps))), smem = x + stages * per_warp * warps;
+    const int stages = max(2, min(8, (budget - x) / (per_warp * warps))), smem = x + stages * per_warp * warps;
     auto kern = few_rows_kernel<MT, CPT, VEC, XRES>;
     // the limit belongs to the function, not to the call: one value, so that no thread's call lowers it under another's
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM_MOST);
@@ -542,31 +557,65 @@ template <int MT, int CPT, bool VEC, bool XRES> int few(const Call& c) {
                               c.bb, c.C, c.ldc, c.M, c.N, c.K, stages);
 }
 
-// Every column of a thread makes its reads of A serve more products (3 rows, N 151,936: 128 us with one, 93 with two, 89 with four;
-// the kernel before it, 32 columns a CTA, took 123), but few columns want the warps (N 896, K 4,864: 14.3, 18.4, 21.0; before 20.6).
-// Rows by sixteen want the registers (N 151,936: 191 us with two, 287 with four; before 417).
+// Rows of A that do not fit whole, cut into blocks that do, where the blocks' CTAs all run side by side: each reads W, but few columns are
+// soon read and few CTAs leave the SMs idle (16 rows, N 256, K 8,960: 23.5 us in four blocks, 58.0 through the rings); -1 where not
+template <int MT> int side_by_side(const Call& c, long long row) {
+    const long long columns = (long long)((c.M + MT - 1) / MT) * c.N, x = min(c.M, MT) * row;
+    if (x <= FEW_X_MOST && columns <= 148 * 8) return few<MT, 1, true, true>(c);
+    if (x <= 94 * 1024 && columns <= 148 * 16) return few<MT, 1, true, true>(c, FEW_SMEM_TWO);
+    if (x <= FEW_X_MOST && columns <= 148 * 16 && c.M > 4) return few<MT, 2, true, true>(c);
+    if constexpr (MT > 1) return side_by_side<MT == 3 ? 2 : MT / 2>(c, row);
+    return -1;
+}
+
+// Which of the two, and with how many columns a lane: from 2,394 shapes of 1 to 16 rows, 8 to 151,936 columns and K 260 to 40,960, weights
+// mostly from memory, and 444 whose rows start off 16-byte boundaries (microseconds).  The first that holds:
+// - N whose CTAs of eight columns all run at once (`PLACES`: their rings bound how many an SM holds) has a ring a CTA where K is too
+//   short to pay for bringing all of A first (8 rows, N 896: K 640 5.2 and 5.2 by warps, K 4,864 25.8 and 19.6), where the rows are
+//   twelve and more (16 rows, N 54, K 2,044: 15.4 and 16.7) or copies are single entries;
+// - rows of A that do not fit whole: blocks of them side by side (above); nine rows and more in two blocks, one after the other, as long as
+//   eight fit and the columns are many (two streams of W, but eight rows leave the SM's shared memory the time for them; 16 rows, N 18,944, K 4,864:
+//   142.6, once 159.4); else through the warps' rings, W once at any K (16 rows, N 4,600, K 18,944: 153.6, a ring a CTA 158.6 with 32 columns; 3 rows,
+//   N 4,200, K 40,960: 104.0 and 220.9); single entries go through a ring a CTA;
+// - just below 148 x 64 columns CTAs of 32 columns, two an SM, leave no SM idle, while the warps' shares are uneven
+//   (1 row, N 9,400, K 896: 6.9, by warps 7.2);
+// - else a ring a warp.  More columns a lane make the reads of A serve more products (8 rows, N 18,944, K 896: 25.8 with one, 18.7 with
+//   two, 17.7 with four), but fewer share few columns more evenly (8 rows, N 3,300, K 896: 7.3, 7.2, 10.7) and leave more warps
+//   beside much of A.  Four take too many registers beyond eight rows and too many bytes a stage beside more than 98 KB of A; one and two
+//   rows gain from them with few columns and a short K only (1 row, N 9,728, K 384: 4.7 with two, 4.3 with four).
+// Three rows have a form of their own: that of four reads a row of A more (10 to 14 % slower below 4,736 columns, 3 to 6 % above where K
+// is below 1,000).
 template <int MT, bool VEC> int few_k(const Call& c) {
-    const long long row = (long long)((c.K + PERIOD - 1) / PERIOD) * PERIOD * 4;       // bytes of a row of A in shared memory
-    if (min(c.M, MT) * row > FEW_X_MOST) {
-        if constexpr (MT > 1) return few_k<MT / 2, VEC>(c);
-        else return few<1, 1, VEC, false>(c);
+    constexpr int CTA_MT = MT == 3 ? 4 : MT;                                           // a ring a CTA has no form of three rows
+    constexpr int PLACES = VEC || MT > 4 ? 148 * 8 * (MT <= 2 ? 4 : MT <= 4 ? 3 : MT <= 8 ? 2 : 1) : 148 * 32 - 1;
+    constexpr int SHORT = MT == 1 ? 1792 : MT == 3 || MT == 4 ? 640 : 1280;
+    const long long row = ((long long)c.K + PERIOD - 1) / PERIOD * PERIOD * 4, x = row * c.M;       // bytes of A in shared memory
+    const bool fits = x <= (MT == 8 && !VEC ? 128 * 1024 : FEW_X_MOST);
+    if (c.N <= PLACES && (!VEC || (fits && (c.K < SHORT || c.M > 11)))) return shared_ring<CTA_MT, 8, 1, 5, VEC>(c);
+    if constexpr (!VEC) {
+        if (!fits) return shared_ring<CTA_MT, 32, 2, 3, VEC>(c);
+    } else {
+        if (!fits) {
+            const int rc = side_by_side<MT>(c, row);
+            if (rc >= 0) return rc;
+            if constexpr (MT == 16) {
+                if (c.N >= 148 * 32 && 8 * row <= FEW_X_MOST)
+                    return c.N >= 148 * 64 && 8 * row <= 98 * 1024 ? few<8, 4, true, true>(c) : few<8, 2, true, true>(c);
+            }
+            return c.N <= 148 * (MT <= 4 ? 28 : MT <= 8 ? 14 : 16) ? few<MT, 1, true, false>(c) : few<MT, 2, true, false>(c);
+        }
+        if constexpr (MT <= 4) {
+            if (c.N <= 148 * 64 && c.N > 148 * (MT > 2 ? 60 : c.K < 1280 ? 40 : 48)) return shared_ring<CTA_MT, 32, 2, 3, VEC>(c);
+        }
     }
-    // four warps a CTA have to fit beside its rows of A
-    const long long room = (FEW_SMEM_MOST - min(c.M, MT) * row) / (4 * 2 * 4 * PERIOD * 4);
     if constexpr (MT <= 8) {
-        if (c.N >= 148 * 64 && room >= 4) return few<MT, 4, VEC, true>(c);
-        if ((c.N < 148 * 32 && c.M <= 8) || room < 2) return few<MT, 1, VEC, true>(c);
+        if (c.N >= 148 * 64 && (MT > 2 ? x <= 98 * 1024 : c.N <= 148 * 84 && c.K <= 1280)) return few<MT, 4, VEC, true>(c);
     }
-    return few<MT, 2, VEC, true>(c);
+    const int one = 148 * (MT == 1 ? 32 : MT <= 8 ? 28 : 16);
+    return c.N <= one || (MT <= 2 && x > 144 * 1024) ? few<MT, 1, VEC, true>(c) : few<MT, 2, VEC, true>(c);
 }
 
 template <bool VEC> int few_m(const Call& c) {
-    // Few columns: their two warps at a time share the copies, which is worth more where K is short, there are one or two rows or
-    // the copies are single entries (K 896, N 896: 1 row 3.6 us, 4.1 by a ring a warp, 3 rows 5.4 and 4.9, 8 rows 6.5 and 7.4; K 4,864:
-    // 1 row 12.5 and 10.0, 3 rows 20.6 and 14.3).
-    if (c.N < 148 * 32 && !(VEC && (c.M <= 2 ? c.M == 1 && c.K >= 2048 && c.N >= 592 : c.K >= (c.M <= 4 ? 640 : 2048))))
-        return c.M <= 1 ? few_columns<1, VEC>(c) : c.M <= 2 ? few_columns<2, VEC>(c) : c.M <= 4 ? few_columns<4, VEC>(c) : c.M <= 8 ?
-               few_columns<8, VEC>(c) : few_columns<16, VEC>(c);
     if (c.M <= 1) return few_k<1, VEC>(c);
     if (c.M <= 2) return few_k<2, VEC>(c);
     if (c.M <= 3) return few_k<3, VEC>(c);

@@ -205,10 +205,12 @@ def test_sgemm_at_the_edges_of_its_tiles(N, K):
         assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6, M
 
 
-@pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9475, 900), (4800, 5200), (600, 41216), (33, 41217)])
+@pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9460, 900), (9475, 900), (4800, 5200), (4800, 4900), (9500, 2900), (33, 9000), (70, 18944), (140, 9000),
+                                 (600, 41216), (3000, 13900), (5000, 18944), (33, 41217), (4739, 12001)])
 def test_sgemm_of_few_rows_with_long_rings(N, K):
-    """Few rows: columns that do not fill a warp's or a CTA's share, a ring that runs on into the next columns, rows of x that fit beside
-    it by sixteen, eight, four or one, or not at all: the bits of the tiles.  Bound: as above."""
+    """Few rows: columns that do not fill a warp's or a CTA's share, a ring that runs on into the next columns, rows of x that stay whole in
+    shared memory, in blocks of eight to one side by side, or go through the rings of the warps or (single entries) of the CTA: the
+    bits of the tiles.  Bound: as above."""
     ops = _ops()
     x, w = _rand((64, K), torch.float32, 18), _rand((N, K), torch.float32, 19, 0.05)
     tiles = torch.empty(64, N, dtype=torch.float32, device=DEV)
@@ -216,9 +218,31 @@ def test_sgemm_of_few_rows_with_long_rings(N, K):
     err = (tiles[:16].double() - x[:16].double() @ w.double().T).abs().max()
     assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
     for M in (16, 13, 9, 8, 5, 4, 3, 2, 1):
-        out = torch.empty(M, N, dtype=torch.float32, device=DEV)
-        ops.sgemm(x[:M], w, None, out)
-        assert torch.equal(out, tiles[:M]), M
+        out = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[:M], w, None, out[:M])
+        assert torch.equal(out[:M], tiles[:M]) and bool((out[M] == 7.0).all()), M
+
+
+def test_sgemm_of_few_rows_reads_the_weights_once_at_any_k():
+    """Sixteen rows whose x does not fit in shared memory: read once, the weights (0.85 GB, nothing of it stays in L2) take what they take
+    for one row, or the multiply-adds of sixteen some four times that; read once a row, or once for every two, eight times or more."""
+    ops = _ops()
+    N, K = 4736, 45000
+    x, w = _rand((16, K), torch.float32, 20), torch.full((N, K), 0.01, dtype=torch.float32, device=DEV)
+    out = torch.empty(16, N, dtype=torch.float32, device=DEV)
+
+    def ms(M):
+        best = float("inf")
+        for _ in range(6):                              # the first is the warm-up
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            ops.sgemm(x[:M], w, None, out[:M])
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert ms(16) < 6 * ms(1)
 
 
 def test_calls_of_several_threads_do_not_change_each_others_limits():
