@@ -161,7 +161,7 @@ __device__ __forceinline__ void few_wait(int stages) {
 // are eight neighbouring lanes.  A row's 16-byte pieces lie at (class, piece ^ class), so that the eight lanes read eight
 // different bank groups.  The weights of the first stages are brought into L2 before the dependency wait; read they are after
 // it, so that they may also be what an earlier kernel of the stream writes.  (One CTA an SM by its shared memory: told so, the compiler takes 69
-// to 255 registers; left alone it kept to 64 and spilled, three rows of K 4,864 to N 896 15.8 us against 13.9.)
+// to 255 registers; left alone it kept to 64 and spilled, three rows of K 4,864 to N 896 15.7 us against 11.2.)
 template <int MT, int CPT, bool VEC, bool XRES>
 __global__ void __launch_bounds__(FEW_WARPS * 32, 1)
 few_rows_kernel(const float* A, int lda, const float* W, int ldw, const void* __restrict__ bias,
@@ -646,21 +646,36 @@ template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC> int ma
 template <bool VEC> int pick(const Call& c) {
     auto tiles = [&](int bm, int bn) { return (long long)((c.M + bm - 1) / bm) * ((c.N + bn - 1) / bn); };
     // A short K (few of the eight classes have a slice) leaves the few rows' lanes and the cluster's CTAs idle: small tiles,
-    // while they are no more than ten an SM (252 rows, N 2,048, K 32: 5.8 us, cluster 16.1; 512 rows, N 8,192, K 16: 14.7 us,
-    // 128 x 64 13.1).  Few rows take longer the more rows and columns they have, the tiles the longer K is (12 rows, N 4,096, K 64:
-    // 4.2 us by tiles, 13.6 by rows; 4 rows, N 512, K 128: 6.2 and 2.4).
+    // while they are no more than ten an SM (252 rows, N 2,048, K 32: 4.4 us, cluster 13.1; 512 rows, N 8,192, K 32: 14.3 us, tiles
+    // of 64 x 64 11.8), by half a slice where K ends in the first (K 8, up to 1,500 tiles: 0.83 to 0.92 of the time).  Few rows take longer the more rows and
+    // columns they have, the tiles the longer K is (12 rows, N 4,096, K 64: 4.2 us by tiles, 13.6 by rows; 4 rows, N 512, K 128: 6.2 and 2.4).
     int rows = 1;
     while (rows < c.M && rows < 32) rows *= 2;
-    if (c.K <= (rows == 32 ? 3 * SLICE : (c.N < 1500 ? 3 : c.N < 4736 ? 10 : 12) * rows))
-        return tiles(32, 32) <= 1500 ? many<32, 32, 4, 4, 32, false, VEC>(c) : many<64, 64, 8, 4, 16, false, VEC>(c);
+    if (c.K <= (rows == 32 ? 3 * SLICE : (c.N < 1500 ? 3 : c.N < 4736 ? 10 : 12) * rows)) {
+        if (tiles(32, 32) > 1500) return many<64, 64, 8, 4, 16, false, VEC>(c);
+        return c.K <= SLICE / 2 ? many<32, 32, 4, 4, 16, false, VEC>(c) : many<32, 32, 4, 4, 32, false, VEC>(c);
+    }
     if (c.M <= 16) return few_m<VEC>(c);
-    // Where tiles of 64 x 64 would not fill the SMs some six times over, a cluster shares their K, as far as its CTAs have slices
-    // (252 rows, N 9,728, K 896, 608 tiles: 130 us, unsplit 137; 512 rows, 1,216 tiles: 250 and 229).  Six of its CTAs fit an SM; where
-    // one round holds all, half tiles may share the SMs more evenly, at some 0.55 of the time each (252 rows, K 4,864: N 896 83 us
-    // against 104; K 896, N 1,152 26.6 and 25.6).
-    if (tiles(64, 64) * PERIOD >= 900LL * (c.K < PERIOD ? c.K : PERIOD)) return many<64, 64, 8, 4, 16, false, VEC>(c);
-    const long long whole = (tiles(64, 64) * CLASSES + 147) / 148, half = (tiles(32, 64) * CLASSES + 147) / 148;
-    return c.M <= 32 || (whole <= 6 && 55 * half < 100 * whole) ? many<32, 64, 4, 4, 16, true, VEC>(c) : many<64, 64, 8, 4, 16, true, VEC>(c);
+    // From 4,600 shapes of 17 to 2,048 rows, K 4 to 20,000.  A cluster shares the K of a tile of 64 x 64 where the tiles alone would not
+    // fill the SMs some five times over.  It is worth less the fewer of its CTAs' slices are whole rounds of the classes (512 rows, N 4,096, 512 tiles: K 512,
+    // 16 slices, 64.1 us and 62.0 unsplit, K 544, 17 slices, 79.4 and 65.5) and the shorter K is, for its two barriers (K 288 57.0 and 36.6).
+    const int slices = (c.K + SLICE - 1) / SLICE, deep = (slices + CLASSES - 1) / CLASSES;
+    const long long t64 = tiles(64, 64), full = slices >= 4 * CLASSES ? 900 : (150LL * slices / deep - 400) * min(c.K, 640) / 640;
+    if (t64 >= (full > 301 ? full : 301) && (t64 > 400 || c.K <= 128 || c.K > 384)) return many<64, 64, 8, 4, 16, false, VEC>(c);
+    // Tiles of 32 x 32 walk a short K alone: their time grows with K, the cluster's with its CTAs (1,000 rows, N 1,000, 256 tiles: K 192
+    // 0.69 of the cluster's time, K 384 0.88, K 512 1.10; 512 rows, N 600, 80 tiles: K 128 0.84, K 192 1.08)
+    if (c.M > 32 && slices <= 12 && t64 > (slices <= 4 ? 18 : min(222, 37 * (slices - 2)))) return many<32, 32, 4, 4, 32, false, VEC>(c);
+    // Split tiles, by how many CTAs of 64 x 64 an SM gets (`whole`; of 32 x 64: `half`, at some 0.55 of the time each).  Half tiles of
+    // whole slices where no SM gets two of them, or more than two but three of 64 x 64 at most: half the barriers, and more bytes on their way from
+    // few CTAs (242 rows, N 707, K 5,900: 85.4 us, 99.8 in tiles of 64 x 64; 900 shapes of up to 55 tiles: 0.8 to 0.9 of the time).  At four, 256
+    // threads a tile (296 rows, N 868, K 14,312: 246 us, 301 with 128).  From there on the SMs are full, and whole tiles read less; half tiles
+    // where they share the SMs more evenly, or those of 64 x 64 leave a fifth of them idle (178 rows, N 278, K 2,309, 120 CTAs: 26.0 us, half tiles
+    // 34.5; 43 rows, N 604, K 11,256, 80 CTAs: 89.3 and 76.7).
+    const long long whole = (t64 * CLASSES + 147) / 148, half = (tiles(32, 64) * CLASSES + 147) / 148;
+    if (half == 1 || (c.M > 32 && half > 2 && whole <= 3)) return many<32, 64, 4, 4, 32, true, VEC>(c);
+    if (c.M > 32 && whole == 4) return many<64, 64, 4, 4, 16, true, VEC>(c);
+    return c.M <= 32 || (half == 2 && t64 < 15) || (whole <= 6 && 55 * half < 100 * whole) ? many<32, 64, 4, 4, 16, true, VEC>(c)
+                                                                             : many<64, 64, 8, 4, 16, true, VEC>(c);
 }
 
 }  // namespace f32gemm

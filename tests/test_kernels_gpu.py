@@ -189,10 +189,10 @@ def test_sgemm_same_at_every_row_count(N, K, pad):
     assert (rows[:, :N].double() - ref).abs().max() < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
 
 
-@pytest.mark.parametrize("N,K", [(65, 47), (60, 112), (1152, 913), (896, 2064), (1000, 2049)])
+@pytest.mark.parametrize("N,K", [(65, 13), (65, 47), (60, 112), (600, 121), (700, 300), (5200, 290), (1152, 913), (896, 2064), (1000, 2049)])
 def test_sgemm_at_the_edges_of_its_tiles(N, K):
-    """Tiles of 32 and 64 rows, whole or with their K shared by a cluster, at their first and last rows and columns and where K ends in
-    either half of a slice: the bits of one row alone.  Bound: a chain of K / 8 products, sums of eight, |x w| of about 0.05."""
+    """Tiles of 32 and 64 rows, whole or with their K shared by a cluster of small or large CTAs, at their first and last rows and columns
+    and where K ends in either half of a slice: the bits of one row alone.  Bound: a chain of K / 8 products, sums of eight, |x w| of about 0.05."""
     ops = _ops()
     x, w = _rand((257, K), torch.float32, 16), _rand((N, K), torch.float32, 17, 0.05)
     one = torch.empty(1, N, dtype=torch.float32, device=DEV)
