@@ -628,7 +628,6 @@ template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC> int ma
     constexpr int smem = many_smem<BM, BN, STEP, SPLIT>();
     static_assert(smem <= 48 * 1024, "");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((c.N + BN - 1) / BN, (c.M + BM - 1) / BM, SPLIT ? CLASSES : 1);
     cfg.blockDim = dim3((BM / TM) * (BN / TN));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
@@ -639,8 +638,15 @@ template <int BM, int BN, int TM, int TN, int STEP, bool SPLIT, bool VEC> int ma
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, many_rows_kernel<BM, BN, TM, TN, STEP, SPLIT, VEC>, c.A, c.lda, c.W, c.ldw, c.bias, c.bb, c.C,
-                                   c.ldc, c.M, c.N, c.K);
+    constexpr long long MOST = 65535LL * BM;       // rows of a launch: what a grid's y takes
+    for (long long m = 0; m < c.M; m += MOST) {
+        const int rows = (int)(c.M - m < MOST ? c.M - m : MOST);
+        cfg.gridDim = dim3((c.N + BN - 1) / BN, (rows + BM - 1) / BM, SPLIT ? CLASSES : 1);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, many_rows_kernel<BM, BN, TM, TN, STEP, SPLIT, VEC>, c.A + m * c.lda, c.lda, c.W, c.ldw,
+                                                 c.bias, c.bb, c.C + m * c.ldc, c.ldc, rows, c.N, c.K);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return 0;
 }
 
 template <bool VEC> int pick(const Call& c) {
@@ -675,7 +681,7 @@ template <bool VEC> int pick(const Call& c) {
     if (half == 1 || (c.M > 32 && half > 2 && whole <= 3)) return many<32, 64, 4, 4, 32, true, VEC>(c);
     if (c.M > 32 && whole == 4) return many<64, 64, 4, 4, 16, true, VEC>(c);
     return c.M <= 32 || (half == 2 && t64 < 15) || (whole <= 6 && 55 * half < 100 * whole) ? many<32, 64, 4, 4, 16, true, VEC>(c)
-                                                                             : many<64, 64, 8, 4, 16, true, VEC>(c);
+                                                                                                 : many<64, 64, 8, 4, 16, true, VEC>(c);
 }
 
 }  // namespace f32gemm

@@ -205,6 +205,20 @@ def test_sgemm_at_the_edges_of_its_tiles(N, K):
         assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6, M
 
 
+def test_sgemm_of_more_rows_than_a_grid_has_tiles():
+    """A grid takes 65,535 tiles of 64 rows; what lies beyond has a launch of its own, with the bits of a small call."""
+    ops = _ops()
+    M, N, K = 65536 * 64 + 70, 5, 12
+    x, w = _rand((M, K), torch.float32, 25), _rand((N, K), torch.float32, 26)
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=DEV)
+    ops.sgemm(x, w, None, out[:M])
+    for rows in (slice(0, 100), slice(65535 * 64 - 50, 65535 * 64 + 50), slice(M - 100, M)):
+        few = torch.empty(100, N, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[rows], w, None, few)
+        assert torch.equal(out[rows], few)
+    assert bool((out[M] == 7.0).all())
+
+
 @pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9460, 900), (9475, 900), (4800, 5200), (4800, 4900), (9500, 2900), (33, 9000), (70, 18944), (140, 9000),
                                  (600, 41216), (3000, 13900), (5000, 18944), (33, 41217), (4739, 12001)])
 def test_sgemm_of_few_rows_with_long_rings(N, K):
