@@ -235,18 +235,65 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 }
             }
         };
-        if constexpr (NTOK >= 32) {                      // K is never split here
+        // this CTA's sums of a split K are in ws: is it the last of its tile's, and so adds them up?
+        auto last_share = [&]() {
+            __threadfence();
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (threadIdx.x == 64) {
+                int* c = counters + blockIdx.y * gridDim.x + blockIdx.x;
+                is_last = atomicAdd(c, 1) == (int)gridDim.z - 1;
+                if (is_last) *c = 0;                                         // ready for the next launch
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (is_last) __threadfence();
+            return is_last != 0;
+        };
+        if constexpr (NTOK >= 32) {
             // Sixteen rows at a time in a loop that stays a loop: a CTA runs its epilogue once, and all rows in straight line code are
             // some 60 KB of instructions that it first has to fetch.  8 experts, all rows unrolled and now: 2 x 672 x 2,048, 256 tokens 72 ->
             // 58 us, 2,048 154 -> 125; 896 x 2,048 without a gate, 64 tokens 45 -> 32, 2,048 153 -> 106; 32 rows at a time 63, 130, 33, 110.
             constexpr int PART = 16;
-            if (go && nkb > 0)
+            const bool split = NTOK <= 64 && gridDim.z > 1;                        // tiles of 128 rows: never
+            constexpr size_t plane = (size_t)NTOK * MOE_TILE_M;                    // one tile's sums of one matrix
+            float* mine = split ? ws + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * gridDim.z * W_TILES * plane + q * 32 + lane : nullptr;
+            auto sums = [&](float (&acc)[W_TILES][PART], int n0) {                 // of this CTA's share of K
+#pragma unroll
+                for (int w = 0; w < W_TILES; ++w)
+                    tmem_load<PART>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + n0, acc[w]);
+            };
+            bool finish = go;
+            if (split && go) {
 #pragma unroll 1
                 for (int n0 = 0; n0 < valid; n0 += PART) {
                     float acc[W_TILES][PART];
+                    if (nkb > 0) sums(acc, n0);
 #pragma unroll
                     for (int w = 0; w < W_TILES; ++w)
-                        tmem_load<PART>(tmem_base + ((uint32_t)(q * 32) << 16) + w * NTOK + n0, acc[w]);
+#pragma unroll
+                        for (int n = 0; n < PART; ++n)
+                            if (n0 + n < valid) mine[((size_t)blockIdx.z * W_TILES + w) * plane + (n0 + n) * MOE_TILE_M] = nkb > 0 ? acc[w][n] : 0.f;
+                }
+                finish = last_share();
+            }
+            if (finish)
+#pragma unroll 1
+                for (int n0 = 0; n0 < valid; n0 += PART) {
+                    float acc[W_TILES][PART];
+                    if (!split) {
+                        sums(acc, n0);
+                    } else {
+#pragma unroll
+                        for (int w = 0; w < W_TILES; ++w)
+#pragma unroll
+                            for (int n = 0; n < PART; ++n) acc[w][n] = 0.f;
+#pragma unroll 1
+                        for (int sp = 0; sp < (int)gridDim.z; ++sp)
+#pragma unroll
+                            for (int w = 0; w < W_TILES; ++w)
+#pragma unroll
+                                for (int n = 0; n < PART; ++n)
+                                    acc[w][n] += n0 + n < valid ? __ldcg(mine + ((size_t)sp * W_TILES + w) * plane + (n0 + n) * MOE_TILE_M) : 0.f;
+                    }
                     finish_rows(acc, n0, std::integral_constant<int, PART>());
                 }
         } else if (go) {
@@ -267,17 +314,8 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
                     for (int n = 0; n < NTOK; ++n)
                         if (n < valid) mine[((size_t)blockIdx.z * W_TILES + w) * plane + n * MOE_TILE_M] = acc[w][n];
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (threadIdx.x == 64) {
-                    int* c = counters + blockIdx.y * gridDim.x + blockIdx.x;
-                    is_last = atomicAdd(c, 1) == (int)gridDim.z - 1;
-                    if (is_last) *c = 0;                                         // ready for the next launch
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                finish = is_last != 0;
+                finish = last_share();
                 if (finish) {
-                    __threadfence();
 #pragma unroll
                     for (int w = 0; w < W_TILES; ++w)
 #pragma unroll
@@ -395,7 +433,7 @@ PRISM_EXPORT int prism_moe_gather(const void* x, long long ldx, const int* offs,
 // out[p] = act(w a_p).
 // shared_rows > 0: an expert that all of them go through rides along: sw [(2) sN, sK] bf16 contiguous, sx [shared_rows, sK]
 // (row stride ldsx), its result at sy (dual: bf16, else float32; row stride ldsy).
-// ksplit > 1: ws of grid tiles * ksplit * (dual 2) * ntok * 128 floats and counters, one int per tile, zero before the
+// ksplit > 1 (not with tiles of 128 rows): ws of grid tiles * ksplit * (dual 2) * ntok * 128 floats and counters, one int per tile, zero before the
 // first launch; tiles: ceil(max(N, sN) / 128) * (token_tiles + ceil(shared_rows / ntok)).
 PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void* w, const int* offs, const int* counts,
                                         const int* row_dst, const float* row_w, int ntok, int token_tiles, int E, int N,
@@ -407,7 +445,7 @@ PRISM_EXPORT int prism_moe_gemm_tcgen05(const void* a, long long lda, const void
     if (E < 1 || K < 8 || K % 8 || lda % 8 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || token_tiles > 65535 ||
         (ntok != 16 && ntok != 32 && ntok != 64 && !(ntok == 128 && dual)))
         return (int)cudaErrorInvalidValue;
-    if (ksplit < 1 || ksplit > (ntok >= 32 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
+    if (ksplit < 1 || ksplit > (ntok > 64 ? 1 : 64) || (ksplit > 1 && (ws == nullptr || counters == nullptr))) return (int)cudaErrorInvalidValue;
     if (shared_rows > 0 && (sw == nullptr || sx == nullptr || sy == nullptr || sN < 1 || sK < 8 || sK % 8 || ldsx % 8 ||
                             ((uintptr_t)sw & 15) || ((uintptr_t)sx & 15) || (!dual && row_dst == nullptr)))
         return (int)cudaErrorInvalidValue;

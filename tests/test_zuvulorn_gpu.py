@@ -607,6 +607,49 @@ def test_experts_in_tiles_of_128_rows(T, W, F, E, top):
         assert float((got - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("ntok", [16, 32, 64])
+@pytest.mark.parametrize("ksplit", [2, 3, 12])
+@pytest.mark.parametrize("form", ["gate", "plain", "down"])
+def test_expert_products_with_k_split_over_ctas(ntok, ksplit, form):
+    """K of 520 (nine blocks of 64) over two, three and twelve CTAs (some without a block) in every tile that can be split, part-filled ones among them: the whole
+    product up to the order of float32 sums (2^-20 of the largest value) and, where the result is bfloat16, its rounding (2^-8 of the
+    value).  The counters are left at zero: a second call gives the same bits."""
+    from prism_b200 import ops
+    E, N, K = 3, 200, 520
+    counts = [ntok + 5, 0, 2 * ntok - 1]
+    offs = [0]
+    for c in counts:
+        offs.append(offs[-1] + -(-c // ntok) * ntok)
+    rows, tiles, dual = offs[-1], offs[-1] // ntok, 1 if form == "gate" else 0
+    g = torch.Generator().manual_seed(ntok + ksplit)
+    a = torch.randn(rows, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E, (1 + dual) * N, K, generator=g) / K ** 0.5).to(torch.bfloat16).to(DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                          # noqa: E731
+    o, c, err = ints(offs), ints(counts), ints([0])
+    live = torch.cat([torch.arange(offs[e], offs[e] + counts[e]) for e in range(E)])
+    dst, by = ints(list(range(rows - 1, -1, -1))), torch.rand(rows, generator=g).to(DEV)
+    xtiles = -(-N // 128)
+    ws = torch.empty(xtiles * tiles * 12 * (1 + dual) * ntok * 128, device=DEV)
+    cnt = torch.zeros(xtiles * tiles, dtype=torch.int32, device=DEV)
+
+    def run(ks):
+        out = torch.zeros(rows, N, dtype=torch.float32 if form == "down" else torch.bfloat16, device=DEV)
+        p = ops._ptr
+        ops._check(ops.lib().prism_moe_gemm_tcgen05(p(a), K, p(w), p(o), p(c), p(dst) if form == "down" else None, p(by) if form == "down" else None,
+                                                    ntok, tiles, E, N, K, dual, ops.MOE_ACTS["relu2" if form == "plain" else "silu"], p(out), N, p(err), None, None, 0, 0,
+                                                    0, 0, None, 0, ks, p(ws), p(cnt), 0.0, ops._stream()), "moe_gemm_tcgen05")
+        return out
+
+    whole, split, again = run(1), run(ksplit), run(ksplit)
+    assert int(err) == 0 and int(cnt.abs().sum()) == 0 and torch.equal(split, again)
+    if form == "down":
+        whole, split = whole.flip(0), split.flip(0)
+    whole, split = whole[live].float(), split[live].float()
+    assert float(whole.abs().max()) > 0.1
+    bound = 2.0 ** -20 * float(whole.abs().max()) + (0.0 if form == "down" else 2.0 ** -7) * whole.abs()
+    assert bool(((split - whole).abs() <= bound).all())
+
+
 # ---------------------------------------------------------------------------------------------------------
 # the model through the engine's step function
 # ---------------------------------------------------------------------------------------------------------
