@@ -173,7 +173,7 @@ def test_sgemm(M, N, K):
                                  (4100, 192), (60, 193), (33, 100)])
 @pytest.mark.parametrize("pad", [0, 1])
 def test_sgemm_same_at_every_row_count(N, K, pad):
-    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone of three sizes with one or several
+    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone of two sizes with one or several
     slices a class, a short K; 16-byte and single copies) adds a row's products in the same order.  Bound: K products of about 0.05, the chains at most K / 8 long."""
     ops = _ops()
     x = _rand((300, K + pad), torch.float32, 6)[:, :K]
@@ -293,26 +293,34 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         assert not errors, (make.__name__, errors[0])
 
 
-@pytest.mark.parametrize("M", [1, 3, 16, 40])
-def test_linear_reads_a_weight_that_was_just_written(M):
-    """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
-    may be read before that kernel has ended.  Bound: two products of K terms, chains of K / 8."""
+@pytest.mark.parametrize("M,N,K", [(1, 3000, 512), (3, 3000, 512), (3, 3000, 896), (16, 3000, 2048), (16, 3000, 512), (8, 9600, 896), (2, 9600, 512), (2, 6000, 896),
+                                   (16, 5000, 3072), (16, 5000, 6000), (12, 200, 4096), (40, 3000, 512)])
+def test_linear_reads_a_weight_that_was_just_written(M, N, K):
+    """A float32 "weight" whose last rows the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``:
+    nothing of it may be read before that kernel has ended.  One shape for each way that few rows go and one for the tiles.  Bound: two
+    products of K terms, chains of K / 8."""
     ops = _ops()
-    N, K = 3000, 512
-    x, b = _rand((M, K), torch.float32, 46), _rand((K, K), torch.float32, 47, 0.05)
-    w = torch.zeros(N, K, dtype=torch.float32, device=DEV)
+    Q, top = 128, max(0, N - (1000 if K <= 2048 else 300))
+    x, b = _rand((M, K), torch.float32, 46), _rand((K, Q), torch.float32, 47, 0.05)
+    old = _rand((N, K), torch.float32, 49)
     outs = []
     for i in range(12):
-        a = _rand((N, K), torch.float32, 48 + i)
+        a = _rand((N - top, Q), torch.float32, 50 + i)
+        w = old.clone()
         y, z = (torch.empty(M, N, dtype=torch.float32, device=DEV) for _ in range(2))
         torch.cuda.synchronize()
-        ops.sgemm(a, b, None, w)                       # 188 tiles of 128 x 64 that release what follows at once
+        # up to 960 tiles of 32 x 32 (eight an SM) or 512 of 64 x 64 (four): all run at once, so that all have released what follows when they begin
+        ops.sgemm(a, b, None, w[top:])
         ops.linear(x, w, None, out=y)
-        ops.sgemm(a, b[:, :], None, w)
+        w[top:].copy_(old[top:])
+        torch.cuda.synchronize()
+        ops.sgemm(a, b, None, w[top:])
         ops.matmul_heads(x[:, None], w[None], z[:, None])
         outs.append((a, y, z))
     for a, y, z in outs:
-        ref = x.double() @ (a.double() @ b.double().T).T
+        w64 = old.double()
+        w64[top:] = a.double() @ b.double().T
+        ref = x.double() @ w64.T
         bound = 2.0 ** -24 * 2 * (K / 8 + 16) * float(ref.abs().max())
         assert float((y.double() - ref).abs().max()) <= bound and torch.equal(y, z)
 
