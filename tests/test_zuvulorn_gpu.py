@@ -269,7 +269,7 @@ def test_second_halves_of_the_low_rank_products_with_their_epilogues(T, R, H, pe
 
 
 @pytest.mark.parametrize("T", [1, 8, 9, 16])
-@pytest.mark.parametrize("blocks, bs, R", [(3, 128, 64), (2, 136, 17), (1, 72, 16), (2, 300, 33), (2, 66, 15)])
+@pytest.mark.parametrize("blocks, bs, R", [(3, 128, 64), (2, 136, 17), (1, 72, 16), (2, 300, 33), (2, 66, 15), (2, 64, 31)])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
 def test_gates_and_low_rank_products_of_few_tokens(T, blocks, bs, R, wdt):
     """The kernels of up to sixteen (eight) tokens, one round of 128 k and more, in 16-byte pieces and entry by entry: every sum has the
