@@ -235,7 +235,7 @@ static int launch_generic(const void* q, int q_stride, int q_head_stride, void* 
     if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
     const size_t smem = (size_t)HPW * ((dk + 7) / 8 * 8 + W * (dv + 2)) * sizeof(float);
     auto kern = attn_generic_kernel<T, MAXD, HPW, W>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    open_smem(kern, smem);
     return (int)launch_kernel(kern, dim3((unsigned)blocks), dim3(W * 32), smem, stream,
         (const T*)q, q_stride, q_head_stride, (T*)out, out_stride, (const T*)kc, k_row_stride, k_head_stride,
         (const T*)vc, v_row_stride, v_head_stride, block_table, bt_width, positions, tok_seg, nh, nkv, dk, dv,

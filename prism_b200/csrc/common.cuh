@@ -76,6 +76,13 @@ inline int& pdl_enabled() {
     return on;
 }
 
+// Shared memory of a launch beyond what needs no asking.  The limit belongs to the kernel and not to a call, and every call sets it: one
+// value, so that no thread's call lowers it under another's (a call that needs more than that still sets its own).
+template <typename... KArgs> inline void open_smem(void (*kern)(KArgs...), size_t smem) {
+    constexpr size_t MOST = 200 * 1024;
+    if (smem > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem > MOST ? smem : MOST));
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  Args... args) {

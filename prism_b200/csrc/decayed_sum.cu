@@ -965,7 +965,7 @@ template <int DVP, int DECAY, bool ROT> static int launch_chunk_out(const DecayC
     const int qs = (a.dk + 15) / 16 * 16 + 8, bs = qs > DVP + 8 ? qs : DVP + 8;
     const size_t smem = (size_t)DS_CHUNK * ((DECAY == PRISM_DS_CHANNEL ? 4 : 2) * qs + 2 * bs) * sizeof(__nv_bfloat16);
     auto kern = decay_chunk_out_kernel<DVP, DECAY, ROT>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    open_smem(kern, smem);
     return (int)launch_kernel(kern, dim3(chunks, a.H), dim3(DS_OUT_THREADS), smem, stream, a);
 }
 
@@ -973,7 +973,7 @@ template <int DECAY, bool ROT> static int launch_chunks(const DecayChunks& a, in
     const int ks = (a.dk + 63) / 64 * 64 + 8, vs = (a.dv + 31) / 32 * 32 + 8;
     const size_t smem = (size_t)DS_CHUNK * 2 * (ks + vs) * sizeof(__nv_bfloat16);
     auto state = decay_chunk_state_kernel<DECAY, ROT>;
-    cudaFuncSetAttribute(state, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    open_smem(state, smem);
     cudaError_t rc = launch_kernel(state, dim3(chunks, a.H), dim3(DS_STATE_THREADS), smem, stream, a);
     if (rc != cudaSuccess) return (int)rc;
     rc = launch_kernel(decay_carry_kernel<DECAY>, dim3((a.dv * a.dk / 4 + 255) / 256, a.H, a.S), dim3(256), 0, stream, a);

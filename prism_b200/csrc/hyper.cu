@@ -171,7 +171,7 @@ PRISM_EXPORT int prism_hyper_norm(const float* x_in, long long in_ss, float* x_o
 #define PRISM_HN(TT, V, SM)                                                                                              \
     do {                                                                                                               \
         auto kern = prism::hyper_norm_kernel<TT, V, SM>;                                                                 \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
+        prism::open_smem(kern, smem);                                                                                  \
         return (int)prism::launch_kernel(kern, dim3(n), dim3(threads), smem, stream, x_in, in_ss, x_out, out_ss, delta, \
                                          delta_dtype == b, nsplit, delta_ss, mix, mix_dtype == b, outw, outw_dtype == b, \
                                          inw, inw_dtype == b, s, weight, weight_dtype == b, eps, rms, (TT*)h, rows, W);  \

@@ -366,7 +366,7 @@ PRISM_EXPORT int prism_moe_route(const float* logits, long long logits_stride, i
     const size_t smem = (size_t)warps * (2 * E + 2 * groups) * sizeof(float);
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     auto kern = prism::moe_route_kernel;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    prism::open_smem(kern, smem);
     return (int)prism::launch_kernel(kern, dim3((T + warps - 1) / warps), dim3(32 * warps), smem, stream, logits, logits_stride,
                                      T, E, top, softmax, renorm, counts, sel_e, sel_w, sel_rank, corr,
                                      corr_dtype == PRISM_DTYPE_BF16, groups, keep, wscale, sum_eps);

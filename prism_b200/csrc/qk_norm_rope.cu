@@ -211,7 +211,7 @@ PRISM_EXPORT int prism_qk_norm_rope_store(const float* q, const float* k, const 
 #define PRISM_QW(TT, V)                                                                                                      \
     do {                                                                                                                     \
         auto kern = prism::qk_norm_whole_kernel<TT, V>;                                                                      \
-        if (row_bytes > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_bytes);  \
+        prism::open_smem(kern, row_bytes);                                                                                   \
         return (int)prism::launch_kernel(kern, dim3(T), dim3(256), row_bytes, stream, q, k, v, ps, wq, qb, wk, kb, eps, freq, rot, \
                                          (TT*)q_out, (TT*)k_plane, (TT*)v_plane, block_table, bt_width, positions, tok_seg, nh, nkv, \
                                          dk, dv, page_size, num_pages, max_pos, err, halves, v_scale);                       \

@@ -1166,7 +1166,7 @@ static int launch_scan(void (*kern)(const ScanArgs), const ScanArgs& a, int vect
     const int per_tok = vectors * a.dkp + a.colsp + 4;
     const size_t smem = ((size_t)a.NBUF * a.TB * per_tok + (a.u != nullptr ? a.dkp : 0)) * sizeof(float);      // BONUS: + u
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    open_smem(kern, smem);
     dim3 grid(a.H, S, (a.dv + a.cols - 1) / a.cols);
     return (int)launch_kernel(kern, grid, dim3((a.cols / cpt * a.L + 31) / 32 * 32 + 32), smem, stream, a);      // + the producer warp
 }
@@ -1200,7 +1200,7 @@ PRISM_EXPORT int prism_conv_unit_gates(const float* proj, long long ps, int ob, 
                             : run(prism::conv_unit_gates_run_kernel<4>);
     }
     auto kern = prism::conv_unit_gates_kernel;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    prism::open_smem(kern, smem);
     const int threads = C >= 2048 ? 1024 : (C >= 512 ? 256 : 128);          // a few channels a thread: their loads are one chain each
     return (int)prism::launch_kernel(kern, dim3(T), dim3(threads), smem, stream, proj, ps, ob, oa, taps,
                                      taps_dtype == PRISM_DTYPE_BF16, K, tail, a_log, a_log_dtype == PRISM_DTYPE_BF16, dt_bias,
@@ -1247,8 +1247,7 @@ PRISM_EXPORT int prism_lowrank_decay(const float* low, long long low_stride, int
     const size_t smem = (size_t)tok * R * sizeof(float);
     if (R < 1 || (size_t)16 * R * sizeof(float) > 200 * 1024 || token_tiles > 65535) return (int)cudaErrorInvalidValue;
     auto kern = tok == 8 ? prism::lowrank_decay_kernel<8> : prism::lowrank_decay_kernel<16>;
-    // the limit belongs to the function, not to the call: one value, so that no thread's call lowers it under another's
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    prism::open_smem(kern, smem);
     return (int)prism::launch_kernel(kern, dim3((N + 127) / 128, token_tiles), dim3(128), smem,
                                      stream, low, low_stride, R, w2t, w0, w0_dtype == PRISM_DTYPE_BF16, N, T, out, out_stride, inner, epi, alog,
                                      alog_dtype == PRISM_DTYPE_BF16, per < 1 ? 1 : per, crate);
@@ -1290,7 +1289,7 @@ PRISM_EXPORT int prism_part_norm_gate(const float* x, const float* gate, long lo
 #define PRISM_PN(TT, V)                                                                                                   \
     do {                                                                                                                  \
         auto kern = part_norm_gate_kernel<TT, V>;                                                                         \
-        if (smem > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
+        open_smem(kern, smem);                                                                                            \
         return (int)launch_kernel(kern, dim3(T, parts), dim3(threads), smem, stream, x, gate, gs, weight, wb, eps, scale, \
                                   parts, w, before, sigmoid_act, (TT*)out, os);                                           \
     } while (0)

@@ -357,7 +357,7 @@ PRISM_EXPORT int prism_add_normed_rmsnorm(float* residual, const void* delta, in
     do {                                                                                                                  \
         using TD = TDx; using TO = TOx;                                                                                   \
         auto plain = prism::add_normed_rmsnorm_kernel<TD, TO>;                                                            \
-        if (smem > 40 * 1024) cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+        prism::open_smem(plain, smem);                                                                                    \
         if (vec && iters == 1)                                                                                            \
             return (int)prism::launch_kernel(prism::add_normed_rmsnorm_vec_kernel<TD, TO, 1>, dim3(nrows), dim3(threads), 0, stream, ARGS); \
         if (vec)                                                                                                          \

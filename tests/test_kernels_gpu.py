@@ -276,6 +276,11 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         out = torch.empty(4, 128, dtype=torch.float32, device=DEV)
         return lambda: ops.lowrank_decay(low, w2t, None, out)
 
+    def norms(width):
+        x, gate = _rand((2, width), torch.float32, 27), _rand((2, width), torch.float32, 28)
+        weight, out = _rand((width,), torch.float32, 29), torch.empty(2, width, dtype=torch.float32, device=DEV)
+        return lambda: ops.part_norm_gate(x, gate, weight, 1e-6, 1, out)
+
     def many(call):
         try:
             for _ in range(3000):
@@ -283,7 +288,7 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         except ops.KernelError as e:
             errors.append(e)
 
-    for make, sizes in ((products, (896, 13568)), (decays, (1600, 3200))):
+    for make, sizes in ((products, (896, 13568)), (decays, (1600, 3200)), (norms, (12000, 40000))):
         threads = [threading.Thread(target=many, args=(make(n),)) for n in sizes * 2]
         for t in threads:
             t.start()
