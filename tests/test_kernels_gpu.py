@@ -173,7 +173,7 @@ def test_sgemm(M, N, K):
                                  (4100, 192), (60, 193), (33, 100)])
 @pytest.mark.parametrize("pad", [0, 1])
 def test_sgemm_same_at_every_row_count(N, K, pad):
-    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone of two sizes with one or several
+    """Every kernel behind ``sgemm`` (few rows, tiles whose K a cluster shares, tiles alone of three sizes with one or several
     slices a class, a short K; 16-byte and single copies) adds a row's products in the same order.  Bound: K products of about 0.05, the chains at most K / 8 long."""
     ops = _ops()
     x = _rand((300, K + pad), torch.float32, 6)[:, :K]
@@ -189,10 +189,10 @@ def test_sgemm_same_at_every_row_count(N, K, pad):
     assert (rows[:, :N].double() - ref).abs().max() < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
 
 
-@pytest.mark.parametrize("N,K", [(65, 13), (65, 47), (60, 112), (600, 121), (700, 300), (5200, 290), (1152, 913), (896, 2064), (1000, 2049)])
+@pytest.mark.parametrize("N,K", [(65, 47), (60, 112), (1152, 913), (896, 2064), (1000, 2049)])
 def test_sgemm_at_the_edges_of_its_tiles(N, K):
-    """Tiles of 32 and 64 rows, whole or with their K shared by a cluster of small or large CTAs, at their first and last rows and columns
-    and where K ends in either half of a slice: the bits of one row alone.  Bound: a chain of K / 8 products, sums of eight, |x w| of about 0.05."""
+    """Tiles of 32 and 64 rows, whole or with their K shared by a cluster, at their first and last rows and columns and where K ends in
+    either half of a slice: the bits of one row alone.  Bound: a chain of K / 8 products, sums of eight, |x w| of about 0.05."""
     ops = _ops()
     x, w = _rand((257, K), torch.float32, 16), _rand((N, K), torch.float32, 17, 0.05)
     one = torch.empty(1, N, dtype=torch.float32, device=DEV)
@@ -203,6 +203,12 @@ def test_sgemm_at_the_edges_of_its_tiles(N, K):
         assert torch.equal(out[:1], one), M
         err = (out.double() - x[:M].double() @ w.double().T).abs().max()
         assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6, M
+
+
+@pytest.mark.parametrize("N,K", [(65, 13), (600, 121), (700, 300), (5200, 290)])
+def test_sgemm_at_the_edges_of_tiles_with_a_short_k(N, K):
+    """K within the first half slice, and of so few slices that a cluster does not share it: as above."""
+    test_sgemm_at_the_edges_of_its_tiles(N, K)
 
 
 def test_sgemm_of_more_rows_than_a_grid_has_tiles():
@@ -219,9 +225,25 @@ def test_sgemm_of_more_rows_than_a_grid_has_tiles():
     assert bool((out[M] == 7.0).all())
 
 
+@pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9475, 900), (4800, 5200), (600, 41216), (33, 41217)])
+def test_sgemm_of_few_rows_with_long_rings(N, K):
+    """Few rows: columns that do not fill a warp's or a CTA's share, a ring that runs on into the next columns, rows of x that fit beside
+    it by sixteen, eight, four or one, or not at all: the bits of the tiles.  Bound: as above."""
+    ops = _ops()
+    x, w = _rand((64, K), torch.float32, 18), _rand((N, K), torch.float32, 19, 0.05)
+    tiles = torch.empty(64, N, dtype=torch.float32, device=DEV)
+    ops.sgemm(x, w, None, tiles)
+    err = (tiles[:16].double() - x[:16].double() @ w.double().T).abs().max()
+    assert err < 2.0 ** -24 * (K / 8 + 16) * (K ** 0.5) * 0.05 * 4 + 1e-6
+    for M in (16, 13, 9, 8, 5, 4, 3, 2, 1):
+        out = torch.empty(M, N, dtype=torch.float32, device=DEV)
+        ops.sgemm(x[:M], w, None, out)
+        assert torch.equal(out, tiles[:M]), M
+
+
 @pytest.mark.parametrize("N,K", [(896, 4864), (601, 2052), (4737, 304), (9460, 900), (9475, 900), (4800, 5200), (4800, 4900), (9500, 2900), (33, 9000), (70, 18944), (140, 9000),
                                  (600, 41216), (3000, 13900), (5000, 18944), (33, 41217), (4739, 12001)])
-def test_sgemm_of_few_rows_with_long_rings(N, K):
+def test_sgemm_of_few_rows_with_x_whole_in_blocks_or_through_the_rings(N, K):
     """Few rows: columns that do not fill a warp's or a CTA's share, a ring that runs on into the next columns, rows of x that stay whole in
     shared memory, in blocks of eight to one side by side, or go through the rings of the warps or (single entries) of the CTA: the
     bits of the tiles.  Bound: as above."""
@@ -298,9 +320,33 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         assert not errors, (make.__name__, errors[0])
 
 
+@pytest.mark.parametrize("M", [1, 3, 16, 40])
+def test_linear_reads_a_weight_that_was_just_written(M):
+    """A float32 "weight" that the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``: nothing of it
+    may be read before that kernel has ended.  Bound: two products of K terms, chains of K / 8."""
+    ops = _ops()
+    N, K = 3000, 512
+    x, b = _rand((M, K), torch.float32, 46), _rand((K, K), torch.float32, 47, 0.05)
+    w = torch.zeros(N, K, dtype=torch.float32, device=DEV)
+    outs = []
+    for i in range(12):
+        a = _rand((N, K), torch.float32, 48 + i)
+        y, z = (torch.empty(M, N, dtype=torch.float32, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        ops.sgemm(a, b, None, w)                       # more CTAs than run at once: the last of them release what follows
+        ops.linear(x, w, None, out=y)
+        ops.sgemm(a, b[:, :], None, w)
+        ops.matmul_heads(x[:, None], w[None], z[:, None])
+        outs.append((a, y, z))
+    for a, y, z in outs:
+        ref = x.double() @ (a.double() @ b.double().T).T
+        bound = 2.0 ** -24 * 2 * (K / 8 + 16) * float(ref.abs().max())
+        assert float((y.double() - ref).abs().max()) <= bound and torch.equal(y, z)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3000, 512), (3, 3000, 512), (3, 3000, 896), (16, 3000, 2048), (16, 3000, 512), (8, 9600, 896), (2, 9600, 512), (2, 6000, 896),
                                    (16, 5000, 3072), (16, 5000, 6000), (12, 200, 4096), (40, 3000, 512)])
-def test_linear_reads_a_weight_that_was_just_written(M, N, K):
+def test_every_form_of_few_rows_reads_a_weight_that_was_just_written(M, N, K):
     """A float32 "weight" whose last rows the kernel right ahead in the stream writes, through ``linear`` and ``matmul_heads``:
     nothing of it may be read before that kernel has ended.  One shape for each way that few rows go and one for the tiles.  Bound: two
     products of K terms, chains of K / 8."""
