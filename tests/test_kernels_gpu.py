@@ -286,7 +286,7 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
     lower it between another's setting and its launch."""
     import threading
     ops = _ops()
-    errors = []
+    errors, keep = [], []
 
     def products(K):
         x, w = _rand((3, K), torch.float32, 21), _rand((896, K), torch.float32, 22)
@@ -303,6 +303,17 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         weight, out = _rand((width,), torch.float32, 29), torch.empty(2, width, dtype=torch.float32, device=DEV)
         return lambda: ops.part_norm_gate(x, gate, weight, 1e-6, 1, out)
 
+    def attentions(dk):
+        q, k, v = (_rand(shape, torch.bfloat16, 30) for shape in ((1, 1, dk), (1, 16, 1, dk), (1, 16, 1, 256)))
+        ints = lambda *n: torch.tensor(n, dtype=torch.int32, device=DEV)                    # noqa: E731
+        table, start, cached, err = ints(0)[None], ints(0, 1), ints(3), ints(0)
+        out = torch.empty(1, 256, dtype=torch.bfloat16, device=DEV)
+        p, call = ops._ptr, ops.lib().prism_attention_masked_bf16
+        args = (p(q), dk, dk, p(out), 256, p(k), dk, dk, p(v), 256, 256, p(table), 1, p(start), p(cached), 1, 1, 1, 1, dk, 256, 16, 1, 0, 0, 0, 0.1,
+                None, 0, 1, 1, None, None, p(err), None, 0, ops._stream())
+        keep.append((q, k, v, table, start, cached, err, out))
+        return lambda: ops._check(call(*args), "attention_masked_bf16")
+
     def many(call):
         try:
             for _ in range(3000):
@@ -310,7 +321,7 @@ def test_calls_of_several_threads_do_not_change_each_others_limits():
         except ops.KernelError as e:
             errors.append(e)
 
-    for make, sizes in ((products, (896, 13568)), (decays, (1600, 3200)), (norms, (12000, 40000))):
+    for make, sizes in ((products, (896, 13568)), (decays, (1600, 3200)), (norms, (12000, 40000)), (attentions, (64, 256))):
         threads = [threading.Thread(target=many, args=(make(n),)) for n in sizes * 2]
         for t in threads:
             t.start()
