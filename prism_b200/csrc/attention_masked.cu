@@ -495,7 +495,7 @@ static int launch_masked(const MaskedAttn& a, int S, int max_q_len, cudaStream_t
     if (SPLITK) smem = std::max(smem, (size_t)(4 * 16 * DVP + 4 * 16 * 2) * sizeof(float));
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     auto kern = attn_masked_kernel<DVP, V_IN_K, SPLITK>;
-    // keys of 340 entries and more want more than open_smem's one value: here it is all there is, for every call
+    // long keys beside long values (256 and 256 in a decode step: 206 KB) want more than open_smem's one value: every call sets all there is
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     dim3 grid(SPLITK ? a.nsplit : (max_q_len + a.tok_per_cta - 1) / a.tok_per_cta, a.nkv * a.hgroups, S);
     const cudaError_t rc = launch_kernel(kern, grid, dim3(MA_THREADS), smem, stream, a);
